@@ -20,10 +20,13 @@
 //     synchronisation is needed and a step stays graph-capturable.  A triangle / edge of at most
 //     half a cell sits in the one bucket of its box centre's cell, a larger (stretched) one in
 //     every cell its box overlaps; the count pass keeps each element's box;
-//   * a query rejects candidates by box overlap before any filter or exact distance, skips
-//     entries of other cells that share its bucket, and keeps the survivors in a sorted
-//     per-vertex / per-edge list (so each pair is reported once);
-//   * forces are gathered per vertex of the current color, one warp per vertex taking the pairs
+//   * a query rejects candidates by box overlap before any filter or exact distance and skips
+//     entries of other cells that share its bucket; a queue per warp hands the survivors to the
+//     exact tests with every lane busy, and the accepted ones end in sorted per-vertex / per-edge
+//     lists (so each pair is reported once);
+//   * the detected pairs are laid out once per detection for the passes that every color runs over
+//     them (entries per vertex for the forces, a flat pair table for the planes);
+//   * forces are gathered per vertex of the current color, one warp per vertex taking its entries
 //     round-robin in a fixed order (own vertex-triangle pairs, then the pairs of each incident
 //     triangle, then the edge-edge pairs of each incident edge) and reduced with xor shuffles, so
 //     results are deterministic;
@@ -38,6 +41,7 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "vbd_self_contact_math.cuh"
@@ -177,31 +181,8 @@ __global__ void grid_fill_kernel(GridArgs a) {
             }
 }
 
-// whether bucket entry (box blo/bhi) belongs to cell (x, y, z): its centre cell, or for a large
-// element any cell its box overlaps
-__device__ __forceinline__ bool in_cell(float4 blo, float4 bhi, float inv, int x, int y, int z) {
-    if (blo.w == 0.f) {
-        const int3 c = center_cell(blo, bhi, inv);
-        return c.x == x && c.y == y && c.z == z;
-    }
-    const CellRange r = cell_range(xyz(blo), xyz(bhi), inv);
-    return x >= r.lo.x && x <= r.hi.x && y >= r.lo.y && y <= r.hi.y && z >= r.lo.z && z <= r.hi.z;
-}
-
 __device__ __forceinline__ bool boxes_overlap(float3 lo, float3 hi, float4 blo, float4 bhi) {
     return !(blo.x > hi.x || bhi.x < lo.x || blo.y > hi.y || bhi.y < lo.y || blo.z > hi.z || bhi.z < lo.z);
-}
-
-// sorted insert without duplicates into row[0..n) of capacity cap; false when full
-__device__ __forceinline__ bool sorted_insert(int* row, int& n, int cap, int x) {
-    int k = 0;
-    while (k < n && row[k] < x) ++k;
-    if (k < n && row[k] == x) return true;
-    if (n >= cap) return false;
-    for (int j = n; j > k; --j) row[j] = row[j - 1];
-    row[k] = x;
-    ++n;
-    return true;
 }
 
 __device__ __forceinline__ bool filtered(const int* off, const int* list, int row, int x) {
@@ -216,9 +197,12 @@ __device__ __forceinline__ bool filtered(const int* off, const int* list, int ro
     return b < list + off[row + 1] && *b == x;
 }
 
-__device__ __forceinline__ bool list_contains(const int* b, const int* e, int x) {
-    for (const int* p = b; p < e; ++p)
-        if (*p == x) return true;
+// whether the list holds u or v (or w): one pass over it
+__device__ __forceinline__ bool list_has(const int* b, const int* e, int u, int v, int w) {
+    for (const int* p = b; p < e; ++p) {
+        const int x = *p;
+        if (x == u || x == v || x == w) return true;
+    }
     return false;
 }
 
@@ -253,39 +237,92 @@ constexpr int kQueryBlock = 128;
 constexpr int kQueryWarps = kQueryBlock / 32;
 constexpr int kEeLanes = 4;  // lanes per edge-edge query (4 measured best of 2, 4, 8)
 
+// ---- candidates -------------------------------------------------------------------------------
+// Both queries run in two halves.  The cheap half -- a staged bucket entry against a lane's query:
+// box overlap, cell ownership -- runs with every lane on its own query and passes a few entries in a
+// hundred; each passed (query, element) pair goes into a small queue of the warp.  The expensive
+// half -- the exact distance, the ring and external filters -- takes 32 queued pairs at a time, one
+// per lane (a lane that evaluated its own pairs as it met them left most of the warp idle).  The
+// distance comes before the filters: most queued pairs are neighbours in the same layer, farther
+// apart than the margin, and the ring filter walks a list.  Accepted partners are appended to their
+// rows through atomic slots; sort_rows_kernel then orders every row, so the lists do not depend on
+// scheduling.  On the folded 1.05 M vertex cloth: edge query 4.59 -> 2.84 ms, vertex query 2.31 -> 1.49 ms.
+struct PairQueue {
+    int2* slots;  // this warp's 64 entries in shared memory
+    int n;        // (warp-uniform)
+};
+
+// queue (q, t) of the lanes with `cand`; 32 queued pairs are handed to `accept`, one per lane
+template <typename Accept>
+__device__ __forceinline__ void queue_push(PairQueue& pq, bool cand, int q, int t, Accept accept) {
+    const int lane = threadIdx.x & 31;
+    const unsigned m = __ballot_sync(0xffffffffu, cand);
+    if (m == 0u) return;
+    if (cand) pq.slots[pq.n + __popc(m & ((1u << lane) - 1u))] = make_int2(q, t);
+    pq.n += __popc(m);
+    if (pq.n >= 32) {
+        __syncwarp();
+        pq.n -= 32;
+        const int2 e = pq.slots[pq.n + lane];
+        __syncwarp();
+        accept(e.x, e.y);
+    }
+}
+
+template <typename Accept>
+__device__ __forceinline__ void queue_flush(PairQueue& pq, Accept accept) {
+    __syncwarp();
+    const int lane = threadIdx.x & 31;
+    if (lane < pq.n) {
+        const int2 e = pq.slots[lane];
+        accept(e.x, e.y);
+    }
+    pq.n = 0;
+}
+
+// Whether the query with cell range q takes the bucket entry (box blo/bhi) in cell (x, y, z): a
+// small element's centre cell; a large one only in the first cell of q that its box occupies, so that
+// every pair is met once
+__device__ __forceinline__ bool owns(const CellRange& q, float4 blo, float4 bhi, float inv, int x, int y, int z) {
+    if (blo.w == 0.f) {
+        const int3 c = center_cell(blo, bhi, inv);
+        return c.x == x && c.y == y && c.z == z;
+    }
+    const CellRange gr = cell_range(xyz(blo), xyz(bhi), inv);
+    if (max(q.lo.x, gr.lo.x) != x || max(q.lo.y, gr.lo.y) != y || max(q.lo.z, gr.lo.z) != z) return false;
+    return x <= gr.hi.x && y <= gr.hi.y && z <= gr.hi.z;
+}
+
 // ---- vertex-triangle candidates ------------------------------------------------------------
 struct VtQuery {
     int i;
-    float3 p, plo, phi;
+    float3 plo, phi;
     CellRange q;
-    int wv;
-    const int *nb, *ne;
-    int* row;
-    int n;
-    bool full;
 };
 
-// the tests after the box pre-filter; appends t to the vertex's sorted list
-__device__ __forceinline__ void vt_accept(const QueryArgs& a, VtQuery& v, int t) {
+// the exact tests of a queued pair; appends t to vertex i's row
+__device__ __forceinline__ void vt_accept(const QueryArgs& a, int i, int t) {
     const int4 tr = a.tri[t];
-    const int i = v.i;
     if (tr.x == i || tr.y == i || tr.z == i) return;
-    if (v.wv >= 0 && tr.w >= 0 && v.wv != tr.w) return;
-    if (list_contains(v.nb, v.ne, tr.x) || list_contains(v.nb, v.ne, tr.y) || list_contains(v.nb, v.ne, tr.z)) return;
-    if (filtered(a.vfilt_off, a.vfilt, i, t)) return;
+    const int wv = a.vworld[i];
+    if (wv >= 0 && tr.w >= 0 && wv != tr.w) return;
+    const float3 p = xyz(a.x[i]);
     float3 bary;
-    const float dist = length(triangle_closest_point(xyz(a.x[tr.x]), xyz(a.x[tr.y]), xyz(a.x[tr.z]), v.p, bary) - v.p);
+    const float dist = length(triangle_closest_point(xyz(a.x[tr.x]), xyz(a.x[tr.y]), xyz(a.x[tr.z]), p, bary) - p);
     if (!(dist < a.margin)) return;
+    if (list_has(a.near + a.near_off[i], a.near + a.near_off[i + 1], tr.x, tr.y, tr.z)) return;
+    if (filtered(a.vfilt_off, a.vfilt, i, t)) return;
     if (a.rest_excl > 0.f) {
         const float3 rp = xyz(a.rest[i]);
         const float dr = length(
             triangle_closest_point(xyz(a.rest[tr.x]), xyz(a.rest[tr.y]), xyz(a.rest[tr.z]), rp, bary) - rp);
         if (dr < a.rest_excl) return;
     }
-    if (!sorted_insert(v.row, v.n, a.vbuf, t)) v.full = true;
+    const int k = atomicAdd(&a.vt_count[i], 1);
+    if (k < a.vbuf) a.vt_list[static_cast<size_t>(i) * a.vbuf + k] = t;
 }
 
-__device__ __forceinline__ void vt_scan_lane(const QueryArgs& a, VtQuery& v) {
+__device__ __forceinline__ void vt_scan_lane(const QueryArgs& a, const VtQuery& v) {
     for (int z = v.q.lo.z; z <= v.q.hi.z; ++z)
         for (int y = v.q.lo.y; y <= v.q.hi.y; ++y)
             for (int x = v.q.lo.x; x <= v.q.hi.x; ++x) {
@@ -295,8 +332,8 @@ __device__ __forceinline__ void vt_scan_lane(const QueryArgs& a, VtQuery& v) {
                 for (int k = b; k < e; ++k) {
                     const float4 blo = a.tri_item_box[2 * k], bhi = a.tri_item_box[2 * k + 1];
                     if (!boxes_overlap(v.plo, v.phi, blo, bhi)) continue;
-                    if (!in_cell(blo, bhi, a.inv_cell, x, y, z)) continue;  // another cell in this bucket
-                    vt_accept(a, v, a.tri_items[k]);
+                    if (!owns(v.q, blo, bhi, a.inv_cell, x, y, z)) continue;  // another cell in this bucket
+                    vt_accept(a, v.i, a.tri_items[k]);
                 }
             }
 }
@@ -319,115 +356,89 @@ __device__ __forceinline__ bool in_range(const CellRange& q, int x, int y, int z
 // entry is staged in shared memory by one lane and tested by all lanes against their own query,
 // so the cheap rejections run with every lane active (a walk per lane diverges: its buckets
 // differ in length from its neighbours').
-__global__ void __launch_bounds__(kQueryBlock) vt_query_kernel(QueryArgs a) {
+__global__ void __launch_bounds__(kQueryBlock) vt_query_kernel(const __grid_constant__ QueryArgs a) {
     __shared__ int s_id[kQueryWarps][32];
     __shared__ float4 s_box[kQueryWarps][64];
+    __shared__ int2 s_queue[kQueryWarps][64];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // consecutive query slots are spatially close vertices (Morton order of the rest shape; the
     // internal vertex order is color-major, so neighbours in it are far apart), which keeps the
     // warp's union of cell ranges small
     const int slot = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = slot < a.V ? a.vt_order[slot] : a.V;
-    const bool active = i < a.V;
     VtQuery v;
     v.i = i;
-    v.n = 0;
-    v.full = false;
     bool ok = false;
-    if (active) {
-        v.p = xyz(a.x[i]);
+    if (i < a.V) {
+        const float3 p = xyz(a.x[i]);
         const float m = a.margin;
-        v.plo = v.p - f3(m, m, m);
-        v.phi = v.p + f3(m, m, m);
+        v.plo = p - f3(m, m, m);
+        v.phi = p + f3(m, m, m);
         // a small triangle within the margin has its box centre within margin + half a cell of p;
         // a large one is in every cell its box overlaps
         const float r = m + 0.5f / a.inv_cell;
-        v.q = cell_range(v.p - f3(r, r, r), v.p + f3(r, r, r), a.inv_cell);
+        v.q = cell_range(p - f3(r, r, r), p + f3(r, r, r), a.inv_cell);
         ok = cell_count(v.q) <= kMaxQueryCells;
-        if (!ok) {
-            atomicAdd(&a.counters[kScGridOverflow], 1u);
-            a.vt_count[i] = 0;
-        } else {
-            v.wv = a.vworld[i];
-            v.nb = a.near + a.near_off[i];
-            v.ne = a.near + a.near_off[i + 1];
-            v.row = a.vt_list + static_cast<size_t>(i) * a.vbuf;
-        }
+        if (!ok) atomicAdd(&a.counters[kScGridOverflow], 1u);
     }
     CellRange u;
     if (!warp_union(ok, v.q, u)) return;
     if (cell_count(u) > kWarpUnionCells) {
         if (ok) vt_scan_lane(a, v);
-    } else {
-        for (int z = u.lo.z; z <= u.hi.z; ++z)
-            for (int y = u.lo.y; y <= u.hi.y; ++y)
-                for (int x = u.lo.x; x <= u.hi.x; ++x) {
-                    const bool mine = ok && in_range(v.q, x, y, z);
-                    if (!__any_sync(0xffffffffu, mine)) continue;
-                    const unsigned h = cell_hash(x, y, z, a.tri_mask);
-                    const int b = a.tri_off[h];
-                    const int cnt = min(b + a.tri_cnt[h], a.tri_cap) - b;
-                    for (int c = 0; c < cnt; c += 32) {
-                        if (c + lane < cnt) {
-                            const int k = b + c + lane;
-                            s_id[w][lane] = a.tri_items[k];
-                            s_box[w][2 * lane] = a.tri_item_box[2 * k];
-                            s_box[w][2 * lane + 1] = a.tri_item_box[2 * k + 1];
-                        }
-                        __syncwarp();
-                        const int mc = min(32, cnt - c);
-                        if (mine) {
-                            for (int t = 0; t < mc; ++t) {
-                                const float4 blo = s_box[w][2 * t], bhi = s_box[w][2 * t + 1];
-                                if (!boxes_overlap(v.plo, v.phi, blo, bhi)) continue;
-                                if (!in_cell(blo, bhi, a.inv_cell, x, y, z)) continue;
-                                vt_accept(a, v, s_id[w][t]);
-                            }
-                        }
-                        __syncwarp();
+        return;
+    }
+    PairQueue pq = {s_queue[w], 0};
+    auto accept = [&](int q, int t) { vt_accept(a, q, t); };
+    for (int z = u.lo.z; z <= u.hi.z; ++z)
+        for (int y = u.lo.y; y <= u.hi.y; ++y)
+            for (int x = u.lo.x; x <= u.hi.x; ++x) {
+                const bool mine = ok && in_range(v.q, x, y, z);
+                if (!__any_sync(0xffffffffu, mine)) continue;
+                const unsigned h = cell_hash(x, y, z, a.tri_mask);
+                const int b = a.tri_off[h];
+                const int cnt = min(b + a.tri_cnt[h], a.tri_cap) - b;
+                for (int c = 0; c < cnt; c += 32) {
+                    if (c + lane < cnt) {
+                        const int k = b + c + lane;
+                        s_id[w][lane] = a.tri_items[k];
+                        s_box[w][2 * lane] = a.tri_item_box[2 * k];
+                        s_box[w][2 * lane + 1] = a.tri_item_box[2 * k + 1];
                     }
+                    __syncwarp();
+                    const int mc = min(32, cnt - c);
+                    for (int t = 0; t < mc; ++t) {
+                        const float4 blo = s_box[w][2 * t], bhi = s_box[w][2 * t + 1];
+                        const bool cand = mine && boxes_overlap(v.plo, v.phi, blo, bhi) &&
+                                          owns(v.q, blo, bhi, a.inv_cell, x, y, z);
+                        queue_push(pq, cand, i, s_id[w][t], accept);
+                    }
+                    __syncwarp();
                 }
-    }
-    if (ok) {
-        a.vt_count[i] = v.n;
-        if (v.full) atomicAdd(&a.counters[kScVtOverflow], 1u);
-    }
+            }
+    queue_flush(pq, accept);
 }
 
 // ---- edge-edge candidates ------------------------------------------------------------------
 // Edge-edge pairs are symmetric: edge e only searches partners g > e and records the pair in both
-// lists through atomic slots; ee_sort_kernel then orders every list.  A partner sits in every
-// cell its box overlaps and is taken only in the first cell of the query range it occupies, so
-// every pair is met exactly once.
+// lists.  A partner sits in every cell its box overlaps and is taken only in the first cell of the
+// query range it occupies (owns).
 struct EeQuery {
     int e;
-    int4 ed;
-    float3 a0, a1, qlo, qhi;
+    float3 qlo, qhi;
     CellRange q;
-    const int *n0b, *n0e, *n1b, *n1e;
 };
 
-__device__ __forceinline__ bool ee_owns(const EeQuery& v, float4 blo, float4 bhi, float inv, int x, int y, int z) {
-    if (blo.w == 0.f) {
-        const int3 c = center_cell(blo, bhi, inv);
-        return c.x == x && c.y == y && c.z == z;
-    }
-    const CellRange gr = cell_range(xyz(blo), xyz(bhi), inv);
-    if (max(v.q.lo.x, gr.lo.x) != x || max(v.q.lo.y, gr.lo.y) != y || max(v.q.lo.z, gr.lo.z) != z) return false;
-    return x <= gr.hi.x && y <= gr.hi.y && z <= gr.hi.z;
-}
-
-__device__ __forceinline__ void ee_accept(const QueryArgs& a, const EeQuery& v, int g) {
+__device__ __forceinline__ void ee_accept(const QueryArgs& a, int e, int g) {
     const int4 gd = a.edge[g];
-    const int4 ed = v.ed;
+    const int4 ed = a.edge[e];
     if (gd.x == ed.x || gd.x == ed.y || gd.y == ed.x || gd.y == ed.y) return;
     if (ed.z >= 0 && gd.z >= 0 && ed.z != gd.z) return;
-    if (list_contains(v.n0b, v.n0e, gd.x) || list_contains(v.n0b, v.n0e, gd.y) || list_contains(v.n1b, v.n1e, gd.x) ||
-        list_contains(v.n1b, v.n1e, gd.y))
-        return;
     float s, t, dist;
-    closest_edge_edge(v.a0, v.a1, xyz(a.x[gd.x]), xyz(a.x[gd.y]), a.par_eps, s, t, dist);
+    closest_edge_edge(xyz(a.x[ed.x]), xyz(a.x[ed.y]), xyz(a.x[gd.x]), xyz(a.x[gd.y]), a.par_eps, s, t, dist);
     if (!(dist < a.margin)) return;
+    if (list_has(a.near + a.near_off[ed.x], a.near + a.near_off[ed.x + 1], gd.x, gd.y, gd.y) ||
+        list_has(a.near + a.near_off[ed.y], a.near + a.near_off[ed.y + 1], gd.x, gd.y, gd.y))
+        return;
     if (a.rest_excl > 0.f) {
         float sr, tr, dr;
         closest_edge_edge(xyz(a.rest[ed.x]), xyz(a.rest[ed.y]), xyz(a.rest[gd.x]), xyz(a.rest[gd.y]), a.par_eps, sr,
@@ -436,7 +447,6 @@ __device__ __forceinline__ void ee_accept(const QueryArgs& a, const EeQuery& v, 
     }
     // the distance of (e, g) and of (g, e) is the same test; record both sides (each side's
     // external filter applies to its own list)
-    const int e = v.e;
     if (!filtered(a.efilt_off, a.efilt, e, g)) {
         const int ke = atomicAdd(&a.ee_count[e], 1);
         if (ke < a.ebuf) a.ee_list[static_cast<size_t>(e) * a.ebuf + ke] = g;
@@ -461,8 +471,8 @@ __device__ __forceinline__ void ee_scan_lane(const QueryArgs& a, const EeQuery& 
                     if (g <= v.e) continue;
                     const float4 blo = a.edge_item_box[2 * k], bhi = a.edge_item_box[2 * k + 1];
                     if (!boxes_overlap(v.qlo, v.qhi, blo, bhi)) continue;
-                    if (!ee_owns(v, blo, bhi, a.inv_cell, x, y, z)) continue;
-                    ee_accept(a, v, g);
+                    if (!owns(v.q, blo, bhi, a.inv_cell, x, y, z)) continue;
+                    ee_accept(a, v.e, g);
                 }
             }
 }
@@ -470,9 +480,10 @@ __device__ __forceinline__ void ee_scan_lane(const QueryArgs& a, const EeQuery& 
 // kEeLanes lanes serve one edge query, so a warp holds 32 / kEeLanes consecutive (spatially
 // adjacent) edges: their union of cell ranges stays close to one query's range, and each lane
 // tests every kEeLanes-th staged entry.  Each (edge, partner) test runs on exactly one lane.
-__global__ void __launch_bounds__(kQueryBlock) ee_query_kernel(QueryArgs a) {
+__global__ void __launch_bounds__(kQueryBlock) ee_query_kernel(const __grid_constant__ QueryArgs a) {
     __shared__ int s_id[kQueryWarps][32];
     __shared__ float4 s_box[kQueryWarps][64];
+    __shared__ int2 s_queue[kQueryWarps][64];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int e = (blockIdx.x * blockDim.x + threadIdx.x) / kEeLanes;
     const int sub = lane % kEeLanes;
@@ -480,23 +491,15 @@ __global__ void __launch_bounds__(kQueryBlock) ee_query_kernel(QueryArgs a) {
     v.e = e;
     bool ok = false;
     if (e < a.E) {
-        v.ed = a.edge[e];
-        v.a0 = xyz(a.x[v.ed.x]);
-        v.a1 = xyz(a.x[v.ed.y]);
+        const int4 ed = a.edge[e];
+        const float3 a0 = xyz(a.x[ed.x]), a1 = xyz(a.x[ed.y]);
         const float m = a.margin;
-        v.qlo = fmin3(v.a0, v.a1) - f3(m, m, m);
-        v.qhi = fmax3(v.a0, v.a1) + f3(m, m, m);
+        v.qlo = fmin3(a0, a1) - f3(m, m, m);
+        v.qhi = fmax3(a0, a1) + f3(m, m, m);
         // every partner sits in all the cells its box overlaps: the query's own cells suffice
         v.q = cell_range(v.qlo, v.qhi, a.inv_cell);
         ok = cell_count(v.q) <= kMaxQueryCells;
-        if (!ok) {
-            if (sub == 0) atomicAdd(&a.counters[kScGridOverflow], 1u);
-        } else {
-            v.n0b = a.near + a.near_off[v.ed.x];
-            v.n0e = a.near + a.near_off[v.ed.x + 1];
-            v.n1b = a.near + a.near_off[v.ed.y];
-            v.n1e = a.near + a.near_off[v.ed.y + 1];
-        }
+        if (!ok && sub == 0) atomicAdd(&a.counters[kScGridOverflow], 1u);
     }
     CellRange u;
     if (!warp_union(ok, v.q, u)) return;
@@ -507,6 +510,8 @@ __global__ void __launch_bounds__(kQueryBlock) ee_query_kernel(QueryArgs a) {
     // partners with id <= the warp's smallest query id are rejected by every lane (g > e): they
     // are dropped while staging, so the lanes only walk the entries that can pass
     const int e_min = __reduce_min_sync(0xffffffffu, ok ? e : INT_MAX);
+    PairQueue pq = {s_queue[w], 0};
+    auto accept = [&](int q, int g) { ee_accept(a, q, g); };
     for (int z = u.lo.z; z <= u.hi.z; ++z)
         for (int y = u.lo.y; y <= u.hi.y; ++y)
             for (int x = u.lo.x; x <= u.hi.x; ++x) {
@@ -529,36 +534,88 @@ __global__ void __launch_bounds__(kQueryBlock) ee_query_kernel(QueryArgs a) {
                     }
                     __syncwarp();
                     const int mc = __popc(kept);
-                    if (mine) {
-                        for (int t = sub; t < mc; t += kEeLanes) {
-                            const int g = s_id[w][t];
-                            if (g <= e) continue;
+                    for (int t0 = 0; t0 < mc; t0 += kEeLanes) {
+                        const int t = t0 + sub;
+                        bool cand = false;
+                        int g = -1;
+                        if (mine && t < mc) {
+                            g = s_id[w][t];
                             const float4 blo = s_box[w][2 * t], bhi = s_box[w][2 * t + 1];
-                            if (!boxes_overlap(v.qlo, v.qhi, blo, bhi)) continue;
-                            if (!ee_owns(v, blo, bhi, a.inv_cell, x, y, z)) continue;
-                            ee_accept(a, v, g);
+                            cand = g > e && boxes_overlap(v.qlo, v.qhi, blo, bhi) &&
+                                   owns(v.q, blo, bhi, a.inv_cell, x, y, z);
                         }
+                        queue_push(pq, cand, e, g, accept);
                     }
                     __syncwarp();
                 }
             }
+    queue_flush(pq, accept);
 }
 
-__global__ void ee_sort_kernel(int E, int* ee_count, int* ee_list, int ebuf) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= E) return;
-    const int n = min(ee_count[e], ebuf);
-    ee_count[e] = n;
-    int* row = ee_list + static_cast<size_t>(e) * ebuf;
-    for (int a = 1; a < n; ++a) {
-        const int x = row[a];
-        int b = a - 1;
-        while (b >= 0 && row[b] > x) {
-            row[b + 1] = row[b];
-            --b;
-        }
-        row[b + 1] = x;
+// Rows in ascending order without duplicates (an element that two colliding cells put into one
+// bucket twice is met twice), kSortLanes lanes per row: every entry's rank is the number of smaller
+// ones.  Rows with a duplicate or more than kSortMax entries (larger buffers) are sorted by one lane.
+// overflow: counts the rows that met more entries than their buffer holds (NULL: already counted).
+// (3.1 M edge rows: 0.67 -> 0.51 ms against an insertion sort by one thread per row.)
+constexpr int kSortLanes = 16;
+constexpr int kSortMax = 4 * kSortLanes;
+
+__global__ void sort_rows_kernel(int rows, int* count, int* list, int buf, unsigned* overflow) {
+    const int r = static_cast<int>((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) / kSortLanes);
+    const int sub = threadIdx.x % kSortLanes;
+    const unsigned group = ((1u << kSortLanes) - 1u) << ((threadIdx.x & 31) & ~(kSortLanes - 1));
+    const int met = r < rows ? count[r] : 0;
+    const int n = min(met, buf);
+    __syncwarp();  // every lane of the row has read the count
+    if (met > buf && sub == 0) {
+        count[r] = buf;
+        if (overflow) atomicAdd(overflow, 1u);
     }
+    if (n < 2) return;  // (uniform over the row's lanes)
+    int* row = list + static_cast<size_t>(r) * buf;
+    bool serial = n > kSortMax;
+    int x[kSortMax / kSortLanes], rank[kSortMax / kSortLanes];
+    if (!serial) {
+        bool dup = false;
+#pragma unroll
+        for (int q = 0; q < kSortMax / kSortLanes; ++q) {
+            const int k = sub + q * kSortLanes;
+            x[q] = k < n ? row[k] : INT_MAX;
+            rank[q] = 0;
+        }
+#pragma unroll
+        for (int p = 0; p < kSortMax / kSortLanes; ++p) {
+            if (p * kSortLanes >= n) break;
+            for (int j = 0; j < kSortLanes; ++j) {
+                if (p * kSortLanes + j >= n) break;
+                const int y = __shfl_sync(group, x[p], j, kSortLanes);
+#pragma unroll
+                for (int q = 0; q < kSortMax / kSortLanes; ++q) {
+                    rank[q] += y < x[q] ? 1 : 0;
+                    dup |= y == x[q] && p * kSortLanes + j < sub + q * kSortLanes && sub + q * kSortLanes < n;
+                }
+            }
+        }
+        serial = __any_sync(group, dup);
+    }
+    if (!serial) {
+#pragma unroll
+        for (int q = 0; q < kSortMax / kSortLanes; ++q)
+            if (sub + q * kSortLanes < n) row[rank[q]] = x[q];
+        return;
+    }
+    if (sub != 0) return;
+    int m = 0;
+    for (int k = 0; k < n; ++k) {
+        const int v = row[k];
+        int b = m - 1;
+        while (b >= 0 && row[b] > v) --b;
+        if (b >= 0 && row[b] == v) continue;
+        for (int j = m; j > b + 1; --j) row[j] = row[j - 1];
+        row[b + 1] = v;
+        ++m;
+    }
+    count[r] = m;
 }
 
 __global__ void tri_reverse_kernel(int V, const int* vt_count, const int* vt_list, int vbuf, int* tv_count,
@@ -591,39 +648,225 @@ __global__ void tri_sort_kernel(int T, int* tv_count, int* tv_list, int tcap) {
     }
 }
 
-// marks every vertex that takes part in a detected pair (the gather skips the others)
-__global__ void mark_contact_vertices_kernel(int V, int E, const int4* tri, const int4* edge, const int* vt_count,
-                                             const int* vt_list, int vbuf, const int* ee_count, unsigned char* flag) {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx < V && vt_count[idx] > 0) {
-        flag[idx] = 1;
-        const int* row = vt_list + static_cast<size_t>(idx) * vbuf;
-        for (int k = 0; k < vt_count[idx]; ++k) {
-            const int4 tr = tri[row[k]];
-            flag[tr.x] = 1;
-            flag[tr.y] = 1;
-            flag[tr.z] = 1;
-        }
+// ---- pair tables -----------------------------------------------------------------------------
+// Built once per detection, read by every color of the iterations until the next one:
+//   * entries: per vertex, the pairs it takes part in (its own vertex-triangle row, then those of its
+//     incident triangles, then of its incident edges), 16 bytes each and contiguous, so that the
+//     force pass streams them with a full warp instead of walking list -> element -> vertex chains
+//     with the few lanes that one short list fills;
+//   * pairs: every pair once, with the part of its division plane that depends on the base positions
+//     only (they stay put between detections).
+// Measured on a 1.05 M vertex cloth with a third of it folded over itself (3.5 M vertex-triangle and
+// 9.8 M edge-edge pairs near the margin), per color: forces 1,696 -> 348 us, planes 1,519 -> 215 us,
+// for 1.4 ms of table building per detection.
+// Offsets come from scans and every slot from a rank inside a sorted row, so the tables do not
+// depend on thread scheduling.  Rows that would end beyond a table's capacity are left out of it
+// and evaluated from the detection lists.
+constexpr long long kEntriesPerVertex = 128;  // capacities, per vertex on average
+constexpr long long kPairsPerVertex = 32;
+constexpr int kIdMask = 0x3fffffff;           // vertex ids are below 2^30
+
+__device__ __forceinline__ int tag(int id, int bits) {
+    return static_cast<int>(static_cast<unsigned>(id) | (static_cast<unsigned>(bits) << 30));
+}
+
+struct TableArgs {
+    int V, E;
+    const float4* x;  // base positions
+    const int4* tri;
+    const int4* edge;
+    const int *inc_t_off, *inc_e_off;
+    const int2 *inc_t, *inc_e;
+    const int *vt_count, *vt_list, *ee_count, *ee_list, *tv_count, *tv_list;
+    int vbuf, ebuf, tcap;
+    bool filtered;    // external edge filters: a pair may be in one of its two rows only
+    long long *ent_cnt, *pair_cnt;
+    const long long *ent_off, *pair_off;
+    int4* ent;
+    int4* pair_ids;
+    float4 *pair_n, *pair_h;
+    long long ent_cap, pair_cap;
+    const int *vcolor, *color_start;
+    int *act_v, *act_vcnt;
+};
+
+// Whether row e of the edge lists reports the pair (e, g): the row of the smaller id does; the
+// other one only when the pair is missing from that row (an external filter, or a full row).
+__device__ __forceinline__ bool ee_reports(const TableArgs& a, int e, int g) {
+    if (g > e) return true;
+    const int n = a.ee_count[g];
+    if (!a.filtered && n < a.ebuf) return false;
+    const int* row = a.ee_list + static_cast<size_t>(g) * a.ebuf;
+    int lo = 0, hi = n;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (row[mid] < e) lo = mid + 1;
+        else hi = mid;
     }
-    if (idx < E && ee_count[idx] > 0) {
-        const int4 ed = edge[idx];
-        flag[ed.x] = 1;
-        flag[ed.y] = 1;
+    return !(lo < n && row[lo] == e);
+}
+
+__global__ void table_count_kernel(TableArgs a) {
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    long long n = 0;
+    int color = -1;
+    if (idx < a.V) {
+        n = a.vt_count[idx];
+        a.pair_cnt[idx] = n;
+        for (int k = a.inc_t_off[idx]; k < a.inc_t_off[idx + 1]; ++k) n += a.tv_count[a.inc_t[k].x];
+        for (int k = a.inc_e_off[idx]; k < a.inc_e_off[idx + 1]; ++k) n += a.ee_count[a.inc_e[k].x];
+        a.ent_cnt[idx] = n;
+        color = n > 0 ? a.vcolor[idx] : -1;
+    }
+    if (idx < a.E) {
+        const int m = a.ee_count[idx];
+        const int* row = a.ee_list + static_cast<size_t>(idx) * a.ebuf;
+        int kept = 0;
+        for (int k = 0; k < m; ++k) kept += ee_reports(a, idx, row[k]) ? 1 : 0;
+        a.pair_cnt[a.V + idx] = kept;
+    }
+    if (idx == 0) {
+        a.ent_cnt[a.V] = 0;
+        a.pair_cnt[a.V + a.E] = 0;
+    }
+    // the color's list of contact-touching vertices: one atomic per warp and color (consecutive
+    // vertices share a color but for the warps at a color's border)
+    const unsigned lanes = __match_any_sync(0xffffffffu, color);
+    if (color >= 0) {
+        const int lane = threadIdx.x & 31, leader = __ffs(lanes) - 1;
+        int base = 0;
+        if (lane == leader) base = atomicAdd(&a.act_vcnt[color], __popc(lanes));
+        base = __shfl_sync(lanes, base, leader);
+        a.act_v[a.color_start[color] + base + __popc(lanes & ((1u << lane) - 1u))] = idx;
     }
 }
 
-// compact lists of the work the per-color passes do: contact-touching vertices by color, and
-// the non-empty vertex-triangle / edge-edge rows (the truncation planes)
-__global__ void compact_kernel(int V, int E, const unsigned char* flag, const int* vcolor, const int* color_start,
-                               const int* vt_count, const int* ee_count, int* act_v, int* act_vcnt, int* act_rows,
-                               int* act_cnt) {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx < V && flag[idx]) {
-        const int c = vcolor[idx];
-        if (c >= 0) act_v[color_start[c] + atomicAdd(&act_vcnt[c], 1)] = idx;
+constexpr int kTableLanes = 8;  // lanes per row / vertex while the tables are filled
+
+// What a division plane (vt_plane, ee_plane) takes from the base positions, in units of the pair's
+// distance h: pair_n = (n / h, reach), pair_h = the four participants' heights over the foot of the
+// second element along n, over h.  The plane will lie at a level l in [0.05, 0.95]; the first
+// element's participants stand at heights of at least about 1, the second's at most about 0, so no
+// displacement crosses it whose component along n / h stays below their distance from those levels
+// (`reach`, less a tenth for rounding).
+__device__ __forceinline__ void write_plane(const TableArgs& a, long long at, int4 ids, float3 n, float h,
+                                            float4 height, int firsts) {
+    const float inv = 1.0f / h;
+    const float4 hh = make_float4(height.x * inv, height.y * inv, height.z * inv, height.w * inv);
+    const float up = firsts == 2 ? fminf(hh.x, hh.y) : hh.x;
+    const float low = firsts == 2 ? fmaxf(hh.z, hh.w) : fmaxf(fmaxf(hh.y, hh.z), hh.w);
+    const float reach = 0.9f * fmaxf(fminf(up - 0.95f, 0.05f - low), 0.f);
+    a.pair_ids[at] = ids;
+    a.pair_n[at] = make_float4(n.x * inv, n.y * inv, n.z * inv, reach);
+    a.pair_h[at] = hh;
+}
+
+__device__ __forceinline__ void vt_plane_base(const TableArgs& a, int i, int4 tr, long long at) {
+    const float3 v = xyz(a.x[i]), t1 = xyz(a.x[tr.x]), t2 = xyz(a.x[tr.y]), t3 = xyz(a.x[tr.z]);
+    float3 bary;
+    const float3 cp = triangle_closest_point(t1, t2, t3, v, bary);
+    const float3 nh = v - cp;
+    const float h = length(nh);
+    const int4 ids = make_int4(i, tr.x, tr.y, tr.z);
+    if (h < 1e-12f) {
+        // the reference's plane has a zero normal here, which shortens nothing
+        a.pair_ids[at] = ids;
+        a.pair_n[at] = make_float4(0.f, 0.f, 0.f, 1.f);
+        a.pair_h[at] = make_float4(0.f, 0.f, 0.f, 0.f);
+        return;
     }
-    if (idx < V && vt_count[idx] > 0) act_rows[atomicAdd(&act_cnt[0], 1)] = idx;
-    if (idx < E && ee_count[idx] > 0) act_rows[V + atomicAdd(&act_cnt[1], 1)] = idx;
+    const float3 n = normalized3(nh);
+    write_plane(a, at, ids, n, h, make_float4(dot(n, nh), dot(n, t1 - cp), dot(n, t2 - cp), dot(n, t3 - cp)), 1);
+}
+
+__device__ __forceinline__ void ee_plane_base(const TableArgs& a, int4 ed, int4 gd, long long at) {
+    const float3 a0 = xyz(a.x[ed.x]), a1 = xyz(a.x[ed.y]), b0 = xyz(a.x[gd.x]), b1 = xyz(a.x[gd.y]);
+    float s, t, dist;
+    closest_edge_edge(a0, a1, b0, b1, 1e-6f, s, t, dist);
+    const float3 c1 = a0 + (a1 - a0) * s, c2 = b0 + (b1 - b0) * t;
+    const float3 nh = c1 - c2;
+    const float h = length(nh);
+    const int4 ids = make_int4(tag(ed.x, 1), ed.y, gd.x, gd.y);
+    if (h < 1e-12f) {
+        // touching edges: the robust normal, heights over the midpoint, no crossing test (reach < 0)
+        const float3 n = robust_edge_pair_normal(a0, a1, b0, b1);
+        const float3 d = c1 * 0.5f + c2 * 0.5f;
+        a.pair_ids[at] = ids;
+        a.pair_n[at] = make_float4(n.x, n.y, n.z, -1.f);
+        a.pair_h[at] = make_float4(dot(n, a0 - d), dot(n, a1 - d), dot(n, b0 - d), dot(n, b1 - d));
+        return;
+    }
+    const float3 n = normalized3(nh);
+    write_plane(a, at, ids, n, h, make_float4(dot(n, a0 - c2), dot(n, a1 - c2), dot(n, b0 - c2), dot(n, b1 - c2)), 2);
+}
+
+__global__ void table_pairs_kernel(TableArgs a) {
+    const int row_id = static_cast<int>((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) / kTableLanes);
+    const int sub = threadIdx.x % kTableLanes, group = (threadIdx.x & 31) / kTableLanes;
+    const bool vt = row_id < a.V, ee = !vt && row_id < a.V + a.E;
+    int n = 0;
+    long long off = 0;
+    if (vt || ee) {
+        off = a.pair_off[row_id];
+        if (a.pair_off[row_id + 1] > off && a.pair_off[row_id + 1] <= a.pair_cap)
+            n = vt ? a.vt_count[row_id] : a.ee_count[row_id - a.V];
+    }
+    if (vt) {
+        const int* row = a.vt_list + static_cast<size_t>(row_id) * a.vbuf;
+        for (int k = sub; k < n; k += kTableLanes) vt_plane_base(a, row_id, a.tri[row[k]], off + k);
+    }
+    // edge rows: ranks of the reported partners inside the row, kTableLanes at a time
+    const int m = __reduce_max_sync(0xffffffffu, ee ? n : 0);
+    const int e = row_id - a.V;
+    int kept = 0;
+    for (int base = 0; base < m; base += kTableLanes) {
+        const int k = base + sub;
+        int g = -1;
+        if (ee && k < n) {
+            g = a.ee_list[static_cast<size_t>(e) * a.ebuf + k];
+            if (!ee_reports(a, e, g)) g = -1;
+        }
+        const unsigned bits = (__ballot_sync(0xffffffffu, g >= 0) >> (group * kTableLanes)) & ((1u << kTableLanes) - 1u);
+        if (g >= 0) ee_plane_base(a, a.edge[e], a.edge[g], off + kept + __popc(bits & ((1u << sub) - 1u)));
+        kept += __popc(bits);
+    }
+}
+
+__global__ void table_entries_kernel(TableArgs a) {
+    const int i = static_cast<int>((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) / kTableLanes);
+    const int sub = threadIdx.x % kTableLanes;
+    if (i >= a.V) return;
+    const long long off = a.ent_off[i], end = a.ent_off[i + 1];
+    if (end == off || end > a.ent_cap) return;
+    int4* out = a.ent + off;
+    const int nv = a.vt_count[i];
+    const int* row = a.vt_list + static_cast<size_t>(i) * a.vbuf;
+    for (int k = sub; k < nv; k += kTableLanes) {
+        const int4 tr = a.tri[row[k]];
+        out[k] = make_int4(tag(tr.x, 3), tr.y, tr.z, i);
+    }
+    out += nv;
+    for (int k = a.inc_t_off[i]; k < a.inc_t_off[i + 1]; ++k) {
+        const int2 ts = a.inc_t[k];
+        const int n = a.tv_count[ts.x];
+        if (n == 0) continue;
+        const int4 tr = a.tri[ts.x];
+        const int* vl = a.tv_list + static_cast<size_t>(ts.x) * a.tcap;
+        for (int j = sub; j < n; j += kTableLanes) out[j] = make_int4(tag(tr.x, ts.y), tr.y, tr.z, vl[j]);
+        out += n;
+    }
+    for (int k = a.inc_e_off[i]; k < a.inc_e_off[i + 1]; ++k) {
+        const int2 es = a.inc_e[k];
+        const int n = a.ee_count[es.x];
+        if (n == 0) continue;
+        const int4 ed = a.edge[es.x];
+        const int* gl = a.ee_list + static_cast<size_t>(es.x) * a.ebuf;
+        for (int j = sub; j < n; j += kTableLanes) {
+            const int4 gd = a.edge[gl[j]];
+            out[j] = make_int4(tag(ed.x, es.y), tag(ed.y, 2), gd.x, gd.y);
+        }
+        out += n;
+    }
 }
 
 __global__ void copy_positions_kernel(int V, const float4* src, float4* cd, float4* disp) {
@@ -649,6 +892,9 @@ struct AccumArgs {
     const int2 *inc_t, *inc_e;
     const int *vt_count, *vt_list, *ee_count, *ee_list, *tv_count, *tv_list;
     int vbuf, ebuf, tcap;
+    const long long* ent_off;
+    const int4* ent;
+    long long ent_cap;
     const int* list;    // the color's contact-touching vertices
     const int* count;   // how many (device)
     float r, ke, kd, mu, eps_u, dt, par_eps;
@@ -665,83 +911,92 @@ __device__ __forceinline__ float lane_sum(float v) {
     return v;
 }
 
-// this lane's share of vertex i's pairs (i < 0: an idle slot that only joins the shuffles)
-__device__ __forceinline__ void accumulate_lane(const AccumArgs& a, int i, int lane, float3& f, Sym3& H) {
-    if (i < 0) return;
-    const float3 p = xyz(a.x[i]), p0 = xyz(a.x0[i]);
+// participant `slot`'s share of the vertex-triangle pair (a, b, c; p), or of the edge pair
+__device__ __forceinline__ bool vt_share(const AccumArgs& a, int ia, int ib, int ic, int ip, int slot, float3& f,
+                                         Sym3& H) {
+    auto start = [&](int k) { return xyz(a.x0[k == 0 ? ia : (k == 1 ? ib : (k == 2 ? ic : ip))]); };
+    return vt_contact_slot(xyz(a.x[ia]), xyz(a.x[ib]), xyz(a.x[ic]), xyz(a.x[ip]), start, slot, a.r, a.ke, a.kd, a.mu,
+                           a.eps_u, a.dt, f, H);
+}
+__device__ __forceinline__ bool ee_share(const AccumArgs& a, int e0, int e1, int g0, int g1, int slot, float3& f,
+                                         Sym3& H) {
+    auto start = [&](int k) { return xyz(a.x0[k == 0 ? e0 : (k == 1 ? e1 : (k == 2 ? g0 : g1))]); };
+    return ee_contact_slot(xyz(a.x[e0]), xyz(a.x[e1]), xyz(a.x[g0]), xyz(a.x[g1]), start, slot, a.r, a.ke, a.kd, a.mu,
+                           a.eps_u, a.dt, a.par_eps, f, H);
+}
+
+// this lane's share of the pairs of a vertex without entries (they did not fit the table), from the
+// detection lists
+__device__ __noinline__ bool accumulate_lists(const AccumArgs& a, int i, int lane, float3& f, Sym3& H) {
+    bool hit = false;
     int idx = 0;  // running pair index of this vertex; the lane takes idx % L == lane
     const int* row = a.vt_list + static_cast<size_t>(i) * a.vbuf;
     const int nv = a.vt_count[i];
     for (int k = lane; k < nv; k += kAccumLanes) {
         const int4 tr = a.tri[row[k]];
-        vt_contact_slot(xyz(a.x[tr.x]), xyz(a.x[tr.y]), xyz(a.x[tr.z]), p, xyz(a.x0[tr.x]), xyz(a.x0[tr.y]),
-                        xyz(a.x0[tr.z]), p0, 3, a.r, a.ke, a.kd, a.mu, a.eps_u, a.dt, f, H);
+        hit |= vt_share(a, tr.x, tr.y, tr.z, i, 3, f, H);
     }
     idx += nv;
     for (int k = a.inc_t_off[i]; k < a.inc_t_off[i + 1]; ++k) {
         const int2 ts = a.inc_t[k];
         const int n = a.tv_count[ts.x];
-        int j = (lane - idx) % kAccumLanes;
-        if (j < 0) j += kAccumLanes;
-        if (j < n) {
-            const int4 tr = a.tri[ts.x];
-            const float3 t0 = xyz(a.x[tr.x]), t1 = xyz(a.x[tr.y]), t2 = xyz(a.x[tr.z]);
-            const float3 s0 = xyz(a.x0[tr.x]), s1 = xyz(a.x0[tr.y]), s2 = xyz(a.x0[tr.z]);
-            const int* vl = a.tv_list + static_cast<size_t>(ts.x) * a.tcap;
-            for (; j < n; j += kAccumLanes) {
-                const int q = vl[j];
-                vt_contact_slot(t0, t1, t2, xyz(a.x[q]), s0, s1, s2, xyz(a.x0[q]), ts.y, a.r, a.ke, a.kd, a.mu,
-                                a.eps_u, a.dt, f, H);
-            }
-        }
+        const int4 tr = a.tri[ts.x];
+        const int* vl = a.tv_list + static_cast<size_t>(ts.x) * a.tcap;
+        for (int j = (lane - idx) & (kAccumLanes - 1); j < n; j += kAccumLanes)
+            hit |= vt_share(a, tr.x, tr.y, tr.z, vl[j], ts.y, f, H);
         idx += n;
     }
     for (int k = a.inc_e_off[i]; k < a.inc_e_off[i + 1]; ++k) {
         const int2 es = a.inc_e[k];
         const int n = a.ee_count[es.x];
-        int j = (lane - idx) % kAccumLanes;
-        if (j < 0) j += kAccumLanes;
-        if (j < n) {
-            const int4 ed = a.edge[es.x];
-            const float3 e0 = xyz(a.x[ed.x]), e1 = xyz(a.x[ed.y]);
-            const float3 e0a = xyz(a.x0[ed.x]), e1a = xyz(a.x0[ed.y]);
-            const int* gl = a.ee_list + static_cast<size_t>(es.x) * a.ebuf;
-            for (; j < n; j += kAccumLanes) {
-                const int4 gd = a.edge[gl[j]];
-                ee_contact_slot(e0, e1, xyz(a.x[gd.x]), xyz(a.x[gd.y]), e0a, e1a, xyz(a.x0[gd.x]), xyz(a.x0[gd.y]),
-                                es.y, a.r, a.ke, a.kd, a.mu, a.eps_u, a.dt, a.par_eps, f, H);
-            }
+        const int4 ed = a.edge[es.x];
+        const int* gl = a.ee_list + static_cast<size_t>(es.x) * a.ebuf;
+        for (int j = (lane - idx) & (kAccumLanes - 1); j < n; j += kAccumLanes) {
+            const int4 gd = a.edge[gl[j]];
+            hit |= ee_share(a, ed.x, ed.y, gd.x, gd.y, es.y, f, H);
         }
         idx += n;
     }
+    return hit;
 }
 
 // Grid-stride over the color's contact-touching vertices (the others hold zero since the last
-// detection).  A warp serves 32 / kAccumLanes vertices per round and the round bound is the same
-// for the whole warp, so every lane joins every shuffle.
-__global__ void accumulate_kernel(AccumArgs a) {
+// detection), a warp per vertex over its contiguous entries.
+__global__ void accumulate_kernel(const __grid_constant__ AccumArgs a) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
     const int n = *a.count;
-    const int lane = threadIdx.x & (kAccumLanes - 1);
-    const int sub = (threadIdx.x & 31) / kAccumLanes;  // vertex slot of this lane in its warp
+    const int lane = threadIdx.x & 31;
     const int warps = gridDim.x * (blockDim.x >> 5);
-    const int warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    constexpr int kVerts = 32 / kAccumLanes;  // vertices per warp and round
-    for (int base = kVerts * warp; base < n; base += kVerts * warps) {
-        const int slot = base + sub;
-        const int i = slot < n ? a.list[slot] : -1;
+    for (int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < n; w += warps) {
+        const int i = a.list[w];
+        const long long off = a.ent_off[i], end = a.ent_off[i + 1];
         float3 f = f3(0.f, 0.f, 0.f);
         Sym3 H = zero_sym();
-        accumulate_lane(a, i, lane, f, H);
-        f.x = lane_sum(f.x);
-        f.y = lane_sum(f.y);
-        f.z = lane_sum(f.z);
-        H.xx = lane_sum(H.xx);
-        H.xy = lane_sum(H.xy);
-        H.xz = lane_sum(H.xz);
-        H.yy = lane_sum(H.yy);
-        H.yz = lane_sum(H.yz);
-        H.zz = lane_sum(H.zz);
-        if (i >= 0 && lane == 0) {
+        bool hit = false;
+        if (end <= a.ent_cap) {
+            for (long long k = off + lane; k < end; k += kAccumLanes) {
+                const int4 en = __ldg(&a.ent[k]);
+                const int slot = static_cast<int>(static_cast<unsigned>(en.x) >> 30);
+                if (en.y >= 0) hit |= vt_share(a, en.x & kIdMask, en.y, en.z, en.w, slot, f, H);
+                else hit |= ee_share(a, en.x & kIdMask, en.y & kIdMask, en.z, en.w, slot, f, H);
+            }
+        } else {
+            hit = accumulate_lists(a, i, lane, f, H);
+        }
+        // most vertices near the margin hold no pair inside the radius: nothing to add up
+        if (__any_sync(0xffffffffu, hit)) {
+            f.x = lane_sum(f.x);
+            f.y = lane_sum(f.y);
+            f.z = lane_sum(f.z);
+            H.xx = lane_sum(H.xx);
+            H.xy = lane_sum(H.xy);
+            H.xz = lane_sum(H.xz);
+            H.yy = lane_sum(H.yy);
+            H.yz = lane_sum(H.yz);
+            H.zz = lane_sum(H.zz);
+        }
+        if (lane == 0) {
             a.f[i] = make_float4(f.x, f.y, f.z, 0.f);
             a.h0[i] = make_float4(H.xx, H.xy, H.xz, H.yy);
             a.h1[i] = make_float4(H.yz, H.zz, 0.f, 0.f);
@@ -755,8 +1010,10 @@ struct TruncArgs {
     const int4* tri;
     const int4* edge;
     const int *vt_count, *vt_list, *ee_count, *ee_list;
-    const int* rows;     // non-empty vertex-triangle rows [0, V), then edge-edge rows [V, V + E)
-    const int* counts;   // [2]
+    const long long* pair_off;  // [V + E + 1]
+    const int4* pair_ids;
+    const float4 *pair_n, *pair_h;
+    long long pair_cap;
     int V, E, vbuf, ebuf;
     float eps, gamma;
     unsigned* ts;
@@ -768,59 +1025,117 @@ __device__ __forceinline__ void ts_min(unsigned* ts, int i, float3 x, float3 dx,
     atomicMin(&ts[i], __float_as_uint(t));
 }
 
-// grid-stride over the non-empty rows (vertex-triangle rows first, then edge-edge rows), kPlanarLanes
-// lanes per row taking its pairs round-robin: the truncation factors are reduced with atomicMin,
-// which does not depend on the order
-constexpr int kPlanarLanes = 16;
-
-__global__ void planar_kernel(TruncArgs a) {
-    const int nv = a.counts[0], ne = a.counts[1];
-    const int sub = threadIdx.x % kPlanarLanes;
-    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) / kPlanarLanes; w < nv + ne;
-         w += gridDim.x * blockDim.x / kPlanarLanes) {
-        if (w < nv) {
-            const int i = a.rows[w];
-            const float3 v = xyz(a.cd[i]), dv = xyz(a.disp[i]);
-            const int* row = a.vt_list + static_cast<size_t>(i) * a.vbuf;
-            for (int k = sub; k < a.vt_count[i]; k += kPlanarLanes) {
-                const int4 tr = a.tri[row[k]];
-                const float3 t1 = xyz(a.cd[tr.x]), t2 = xyz(a.cd[tr.y]), t3 = xyz(a.cd[tr.z]);
-                const float3 d1 = xyz(a.disp[tr.x]), d2 = xyz(a.disp[tr.y]), d3 = xyz(a.disp[tr.z]);
-                float3 n, d;
-                const int dummy = vt_plane(v, dv, t1, d1, t2, d2, t3, d3, n, d);
-                if (!(dummy & 1)) ts_min(a.ts, i, v, dv, n, d, a.eps, a.gamma);
-                if (!(dummy & 2)) ts_min(a.ts, tr.x, t1, d1, n, d, a.eps, a.gamma);
-                if (!(dummy & 4)) ts_min(a.ts, tr.y, t2, d2, n, d, a.eps, a.gamma);
-                if (!(dummy & 8)) ts_min(a.ts, tr.z, t3, d3, n, d, a.eps, a.gamma);
-            }
-        } else {
-            const int e = a.rows[a.V + (w - nv)];
-            const int4 ed = a.edge[e];
-            const float3 a0 = xyz(a.cd[ed.x]), a1 = xyz(a.cd[ed.y]);
-            const float3 da0 = xyz(a.disp[ed.x]), da1 = xyz(a.disp[ed.y]);
-            const int* row = a.ee_list + static_cast<size_t>(e) * a.ebuf;
-            for (int k = sub; k < a.ee_count[e]; k += kPlanarLanes) {
-                const int4 gd = a.edge[row[k]];
-                const float3 b0 = xyz(a.cd[gd.x]), b1 = xyz(a.cd[gd.y]);
-                const float3 db0 = xyz(a.disp[gd.x]), db1 = xyz(a.disp[gd.y]);
-                float3 n, d;
-                const int dummy = ee_plane(a0, da0, a1, da1, b0, db0, b1, db1, n, d);
-                if (!(dummy & 1)) ts_min(a.ts, ed.x, a0, da0, n, d, a.eps, a.gamma);
-                if (!(dummy & 2)) ts_min(a.ts, ed.y, a1, da1, n, d, a.eps, a.gamma);
-                if (!(dummy & 4)) ts_min(a.ts, gd.x, b0, db0, n, d, a.eps, a.gamma);
-                if (!(dummy & 8)) ts_min(a.ts, gd.y, b1, db1, n, d, a.eps, a.gamma);
-            }
+// one row of the detection lists (rows that did not fit the pair table)
+__device__ __noinline__ void planar_row(const TruncArgs& a, int w) {
+    if (w < a.V) {
+        const int i = w;
+        const float3 v = xyz(a.cd[i]), dv = xyz(a.disp[i]);
+        const int* row = a.vt_list + static_cast<size_t>(i) * a.vbuf;
+        for (int k = 0; k < a.vt_count[i]; ++k) {
+            const int4 tr = a.tri[row[k]];
+            const float3 t1 = xyz(a.cd[tr.x]), t2 = xyz(a.cd[tr.y]), t3 = xyz(a.cd[tr.z]);
+            const float3 d1 = xyz(a.disp[tr.x]), d2 = xyz(a.disp[tr.y]), d3 = xyz(a.disp[tr.z]);
+            float3 n, d;
+            const int dummy = vt_plane(v, dv, t1, d1, t2, d2, t3, d3, n, d);
+            if (!(dummy & 1)) ts_min(a.ts, i, v, dv, n, d, a.eps, a.gamma);
+            if (!(dummy & 2)) ts_min(a.ts, tr.x, t1, d1, n, d, a.eps, a.gamma);
+            if (!(dummy & 4)) ts_min(a.ts, tr.y, t2, d2, n, d, a.eps, a.gamma);
+            if (!(dummy & 8)) ts_min(a.ts, tr.z, t3, d3, n, d, a.eps, a.gamma);
         }
+        return;
+    }
+    const int e = w - a.V;
+    const int4 ed = a.edge[e];
+    const float3 a0 = xyz(a.cd[ed.x]), a1 = xyz(a.cd[ed.y]);
+    const float3 da0 = xyz(a.disp[ed.x]), da1 = xyz(a.disp[ed.y]);
+    const int* row = a.ee_list + static_cast<size_t>(e) * a.ebuf;
+    for (int k = 0; k < a.ee_count[e]; ++k) {
+        const int4 gd = a.edge[row[k]];
+        const float3 b0 = xyz(a.cd[gd.x]), b1 = xyz(a.cd[gd.y]);
+        const float3 db0 = xyz(a.disp[gd.x]), db1 = xyz(a.disp[gd.y]);
+        float3 n, d;
+        const int dummy = ee_plane(a0, da0, a1, da1, b0, db0, b1, db1, n, d);
+        if (!(dummy & 1)) ts_min(a.ts, ed.x, a0, da0, n, d, a.eps, a.gamma);
+        if (!(dummy & 2)) ts_min(a.ts, ed.y, a1, da1, n, d, a.eps, a.gamma);
+        if (!(dummy & 4)) ts_min(a.ts, gd.x, b0, db0, n, d, a.eps, a.gamma);
+        if (!(dummy & 8)) ts_min(a.ts, gd.y, b1, db1, n, d, a.eps, a.gamma);
     }
 }
 
-// apply_truncation_ts: disp *= t, clamp |disp| to max_disp, pos = cd + disp; t is reset to 1
+// One pair per thread, grid-stride: the division planes of vt_plane / ee_plane from the table's
+// base-position part (write_plane) and the current displacements.  Most pairs end at the reach test,
+// with 32 bytes of table read.  The ratios are reduced with atomicMin, which does not depend on
+// the order.
+__global__ void planar_kernel(const __grid_constant__ TruncArgs a) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
+    const int rows = a.V + a.E;
+    const long long total = a.pair_off[rows];
+    const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
+    const long long first = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    long long fit = total;
+    int slow = rows;  // first row that is not in the table
+    if (total > a.pair_cap) {
+        int lo = 0, hi = rows;
+        while (lo < hi) {
+            const int mid = lo + ((hi - lo) >> 1);
+            if (a.pair_off[mid + 1] <= a.pair_cap) lo = mid + 1;
+            else hi = mid;
+        }
+        slow = lo;
+        fit = a.pair_off[lo];
+    }
+    for (long long k = first; k < fit; k += stride) {
+        const int4 id = __ldg(&a.pair_ids[k]);
+        const float4 nn = __ldg(&a.pair_n[k]);
+        const bool ee = (id.x >> 30) != 0;
+        const int i0 = id.x & kIdMask;
+        const float3 n = xyz(nn);
+        const float q0 = dot(n, xyz(a.disp[i0])), q1 = dot(n, xyz(a.disp[id.y])), q2 = dot(n, xyz(a.disp[id.z])),
+                    q3 = dot(n, xyz(a.disp[id.w]));
+        const bool touching = nn.w < 0.f;
+        if (fmaxf(fmaxf(fabsf(q0), fabsf(q1)), fmaxf(fabsf(q2), fabsf(q3))) < nn.w) continue;
+        const float first_side = fmaxf(ee ? fmaxf(-q0, -q1) : -q0, 0.f);
+        const float second_side = fmaxf(ee ? fmaxf(q2, q3) : fmaxf(fmaxf(q1, q2), q3), 0.f);
+        const float both = first_side + second_side;
+        if (both == 0.f && !touching) continue;
+        const float4 hh = __ldg(&a.pair_h[k]);
+        float l = second_side / both;
+        l = l < 0.05f ? 0.05f : (l > 0.95f ? 0.95f : l);
+        if (touching) l = 0.f;
+        const float h = rsqrtf(dot(n, n));  // back to lengths for the parallel tests
+        const float far = ee ? 1e-6f : 1e-8f;
+        const float q[4] = {q0, q1, q2, q3};
+        const float height[4] = {hh.x, hh.y, hh.z, hh.w};
+        const int who[4] = {i0, id.y, id.z, id.w};
+        const int firsts = ee ? 2 : 1;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float t = (l - height[j]) / q[j];
+            if (!touching) {
+                if ((j < firsts ? first_side : second_side) == 0.f || fabsf(q[j]) * h < 1e-6f) continue;
+                if (!(t >= -1e-8f && t <= 1.f + far)) continue;
+            }
+            if (fabsf(q[j]) * h < a.eps || t < 0.f) continue;  // ratio 1
+            atomicMin(&a.ts[who[j]], __float_as_uint(clamp01f(fminf(t * a.gamma, t - 1e-3f))));
+        }
+    }
+    for (long long w = slow + first; w < rows; w += stride) planar_row(a, static_cast<int>(w));
+}
+
+// apply_truncation_ts: disp *= t, clamp |disp| to max_disp, pos = cd + disp; t is reset to 1.  Only
+// where something changed: the vertices [b, e) (the color just solved, or all) and those with t < 1.
+// (The others' displacements and positions already are what the same arithmetic would write.)
 __global__ void apply_truncation_kernel(int V, const float4* cd, float4* disp, float4* pos, unsigned* ts,
-                                        float max_disp) {
+                                        float max_disp, int b, int e) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= V) return;
     const float t = __uint_as_float(ts[i]);
-    ts[i] = __float_as_uint(1.0f);
+    const bool cut = t != 1.0f;
+    if (!cut && (i < b || i >= e)) return;
+    if (cut) ts[i] = __float_as_uint(1.0f);
     const float4 d4 = disp[i];
     float3 d = f3(d4.x * t, d4.y * t, d4.z * t);
     const float l = length(d);
@@ -908,8 +1223,8 @@ void self_contact_free(SelfContact& sc) {
                     sc.near,     sc.rest,     sc.vt_order,     sc.tri_cnt,   sc.tri_off,  sc.tri_cur,    sc.tri_items, sc.edge_cnt,
                     sc.edge_off, sc.edge_cur, sc.edge_items, sc.scan_tmp, sc.vt_count,  sc.vt_list,   sc.ee_count,
                     sc.ee_list,  sc.tv_count, sc.tv_list,   sc.cd,       sc.sc_f,       sc.sc_h0,     sc.sc_h1,
-                    sc.ts,       sc.counters, sc.vworld,    sc.tri_box,  sc.edge_box,   sc.flag,      sc.tri_item_box, sc.edge_item_box, sc.vfilt_off, sc.vfilt, sc.efilt_off, sc.efilt, sc.color_start, sc.vcolor,
-                    sc.act_v,    sc.act_vcnt, sc.act_rows, sc.act_cnt};
+                    sc.ts,       sc.counters, sc.vworld,    sc.tri_box,  sc.edge_box,   sc.tri_item_box, sc.edge_item_box, sc.vfilt_off, sc.vfilt, sc.efilt_off, sc.efilt, sc.color_start, sc.vcolor,
+                    sc.act_v,    sc.act_vcnt, sc.ent_cnt, sc.ent_off, sc.ent, sc.pair_cnt, sc.pair_off, sc.pair_ids, sc.pair_n, sc.pair_h};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     SelfContact empty;
@@ -1077,11 +1392,19 @@ int self_contact_create(const VbdModelImpl& m, const SelfContactParams& p, SelfC
     az(reinterpret_cast<void**>(&sc.edge_box), 2 * static_cast<size_t>(std::max(E, 1)) * sizeof(float4));
     az(reinterpret_cast<void**>(&sc.tri_item_box), 2 * static_cast<size_t>(sc.tri_items_cap) * sizeof(float4));
     az(reinterpret_cast<void**>(&sc.edge_item_box), 2 * static_cast<size_t>(sc.edge_items_cap) * sizeof(float4));
-    az(reinterpret_cast<void**>(&sc.flag), static_cast<size_t>(V));
     az(reinterpret_cast<void**>(&sc.act_v), static_cast<size_t>(V) * sizeof(int));
     az(reinterpret_cast<void**>(&sc.act_vcnt), static_cast<size_t>(std::max(m.C, 1)) * sizeof(int));
-    az(reinterpret_cast<void**>(&sc.act_rows), static_cast<size_t>(V + E) * sizeof(int));
-    az(reinterpret_cast<void**>(&sc.act_cnt), 2 * sizeof(int));
+    const size_t rows = static_cast<size_t>(V) + E + 1;
+    sc.ent_cap = kEntriesPerVertex * V;
+    sc.pair_cap = kPairsPerVertex * V;
+    az(reinterpret_cast<void**>(&sc.ent_cnt), (static_cast<size_t>(V) + 1) * sizeof(long long));
+    az(reinterpret_cast<void**>(&sc.ent_off), (static_cast<size_t>(V) + 1) * sizeof(long long));
+    az(reinterpret_cast<void**>(&sc.ent), static_cast<size_t>(sc.ent_cap) * sizeof(int4));
+    az(reinterpret_cast<void**>(&sc.pair_cnt), rows * sizeof(long long));
+    az(reinterpret_cast<void**>(&sc.pair_off), rows * sizeof(long long));
+    az(reinterpret_cast<void**>(&sc.pair_ids), static_cast<size_t>(sc.pair_cap) * sizeof(int4));
+    az(reinterpret_cast<void**>(&sc.pair_n), static_cast<size_t>(sc.pair_cap) * sizeof(float4));
+    az(reinterpret_cast<void**>(&sc.pair_h), static_cast<size_t>(sc.pair_cap) * sizeof(float4));
     az(reinterpret_cast<void**>(&sc.vt_count), static_cast<size_t>(V) * sizeof(int));
     az(reinterpret_cast<void**>(&sc.vt_list), static_cast<size_t>(V) * p.vertex_buffer * sizeof(int));
     az(reinterpret_cast<void**>(&sc.ee_count), static_cast<size_t>(E) * sizeof(int));
@@ -1098,9 +1421,12 @@ int self_contact_create(const VbdModelImpl& m, const SelfContactParams& p, SelfC
         size_t b1 = 0, b2 = 0;
         cudaError_t e1 = cub::DeviceScan::ExclusiveSum(nullptr, b1, sc.tri_cnt, sc.tri_off, static_cast<int>(tn));
         cudaError_t e2 = cub::DeviceScan::ExclusiveSum(nullptr, b2, sc.edge_cnt, sc.edge_off, static_cast<int>(en));
+        size_t b3 = 0;
+        cudaError_t e3 = cub::DeviceScan::ExclusiveSum(nullptr, b3, sc.pair_cnt, sc.pair_off, static_cast<int>(rows));
         if (e1 != cudaSuccess) rc = cuda_fail(e1, "cub::DeviceScan::ExclusiveSum (size query)");
         if (!rc && e2 != cudaSuccess) rc = cuda_fail(e2, "cub::DeviceScan::ExclusiveSum (size query)");
-        sc.scan_bytes = std::max(b1, b2);
+        if (!rc && e3 != cudaSuccess) rc = cuda_fail(e3, "cub::DeviceScan::ExclusiveSum (size query)");
+        sc.scan_bytes = std::max(std::max(b1, b2), b3);
         az(&sc.scan_tmp, sc.scan_bytes);
     }
     if (!rc && V > 0) {
@@ -1227,39 +1553,99 @@ int self_contact_detect(const VbdModelImpl& m, SelfContact& sc, const float4* po
     q.ee_count = sc.ee_count;
     q.ee_list = sc.ee_list;
     q.counters = sc.counters;
+    auto sort_rows = [&](int rows, int* count, int* list, int buf, unsigned* overflow) {
+        const long long threads = static_cast<long long>(rows) * kSortLanes;
+        sort_rows_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, st>>>(rows, count, list, buf, overflow);
+    };
+    VBD_CUDA_TRY(cudaMemsetAsync(sc.vt_count, 0, static_cast<size_t>(V) * sizeof(int), st));
     if (T > 0) {
         vt_query_kernel<<<(V + kQueryBlock - 1) / kQueryBlock, kQueryBlock, 0, st>>>(q);
+        VBD_CUDA_TRY(cudaGetLastError());
+        sort_rows(V, sc.vt_count, sc.vt_list, sc.p.vertex_buffer, sc.counters + kScVtOverflow);
         VBD_CUDA_TRY(cudaGetLastError());
         tri_reverse_kernel<<<(V + 255) / 256, 256, 0, st>>>(V, sc.vt_count, sc.vt_list, sc.p.vertex_buffer,
                                                             sc.tv_count, sc.tv_list, sc.tcap, sc.counters);
         VBD_CUDA_TRY(cudaGetLastError());
         tri_sort_kernel<<<(T + 255) / 256, 256, 0, st>>>(T, sc.tv_count, sc.tv_list, sc.tcap);
         VBD_CUDA_TRY(cudaGetLastError());
-    } else {
-        VBD_CUDA_TRY(cudaMemsetAsync(sc.vt_count, 0, static_cast<size_t>(V) * sizeof(int), st));
     }
     if (E > 0) {
         VBD_CUDA_TRY(cudaMemsetAsync(sc.ee_count, 0, static_cast<size_t>(E) * sizeof(int), st));
         const long long ee_threads = static_cast<long long>(E) * kEeLanes;
         ee_query_kernel<<<static_cast<unsigned>((ee_threads + kQueryBlock - 1) / kQueryBlock), kQueryBlock, 0, st>>>(q);
         VBD_CUDA_TRY(cudaGetLastError());
-        ee_sort_kernel<<<(E + 255) / 256, 256, 0, st>>>(E, sc.ee_count, sc.ee_list, sc.p.edge_buffer);
+        sort_rows(E, sc.ee_count, sc.ee_list, sc.p.edge_buffer, nullptr);
         VBD_CUDA_TRY(cudaGetLastError());
     }
-    VBD_CUDA_TRY(cudaMemsetAsync(sc.flag, 0, static_cast<size_t>(V), st));
-    const int nm = std::max(V, E);
-    mark_contact_vertices_kernel<<<(nm + 255) / 256, 256, 0, st>>>(V, E, sc.tri, sc.edge, sc.vt_count, sc.vt_list,
-                                                                   sc.p.vertex_buffer, sc.ee_count, sc.flag);
-    VBD_CUDA_TRY(cudaGetLastError());
-    VBD_CUDA_TRY(cudaMemsetAsync(sc.act_vcnt, 0, static_cast<size_t>(std::max(sc.C, 1)) * sizeof(int), st));
-    VBD_CUDA_TRY(cudaMemsetAsync(sc.act_cnt, 0, 2 * sizeof(int), st));
-    compact_kernel<<<(nm + 255) / 256, 256, 0, st>>>(V, E, sc.flag, sc.vcolor, sc.color_start, sc.vt_count,
-                                                     sc.ee_count, sc.act_v, sc.act_vcnt, sc.act_rows, sc.act_cnt);
-    VBD_CUDA_TRY(cudaGetLastError());
     // vertices that touch no pair keep a zero contact term until the next detection
     VBD_CUDA_TRY(cudaMemsetAsync(sc.sc_f, 0, static_cast<size_t>(V) * sizeof(float4), st));
     VBD_CUDA_TRY(cudaMemsetAsync(sc.sc_h0, 0, static_cast<size_t>(V) * sizeof(float4), st));
     VBD_CUDA_TRY(cudaMemsetAsync(sc.sc_h1, 0, static_cast<size_t>(V) * sizeof(float4), st));
+    VBD_CUDA_TRY(cudaMemsetAsync(sc.act_vcnt, 0, static_cast<size_t>(std::max(sc.C, 1)) * sizeof(int), st));
+    TableArgs t;
+    t.V = V;
+    t.E = E;
+    t.x = sc.cd;
+    t.tri = sc.tri;
+    t.edge = sc.edge;
+    t.inc_t_off = sc.inc_t_off;
+    t.inc_e_off = sc.inc_e_off;
+    t.inc_t = sc.inc_t;
+    t.inc_e = sc.inc_e;
+    t.vt_count = sc.vt_count;
+    t.vt_list = sc.vt_list;
+    t.ee_count = sc.ee_count;
+    t.ee_list = sc.ee_list;
+    t.tv_count = sc.tv_count;
+    t.tv_list = sc.tv_list;
+    t.vbuf = sc.p.vertex_buffer;
+    t.ebuf = sc.p.edge_buffer;
+    t.tcap = sc.tcap;
+    t.filtered = sc.efilt_off != nullptr;
+    t.ent_cnt = sc.ent_cnt;
+    t.pair_cnt = sc.pair_cnt;
+    t.ent_off = sc.ent_off;
+    t.pair_off = sc.pair_off;
+    t.ent = sc.ent;
+    t.pair_ids = sc.pair_ids;
+    t.pair_n = sc.pair_n;
+    t.pair_h = sc.pair_h;
+    t.ent_cap = sc.ent_cap;
+    t.pair_cap = sc.pair_cap;
+    t.vcolor = sc.vcolor;
+    t.color_start = sc.color_start;
+    t.act_v = sc.act_v;
+    t.act_vcnt = sc.act_vcnt;
+    const int nm = std::max(V, E);
+    table_count_kernel<<<(nm + 255) / 256, 256, 0, st>>>(t);
+    VBD_CUDA_TRY(cudaGetLastError());
+    size_t bytes = sc.scan_bytes;
+    VBD_CUDA_TRY(cub::DeviceScan::ExclusiveSum(sc.scan_tmp, bytes, sc.ent_cnt, sc.ent_off, V + 1, st));
+    bytes = sc.scan_bytes;
+    VBD_CUDA_TRY(cub::DeviceScan::ExclusiveSum(sc.scan_tmp, bytes, sc.pair_cnt, sc.pair_off, V + E + 1, st));
+    auto blocks = [](long long rows) { return static_cast<unsigned>((rows * kTableLanes + 127) / 128); };
+    table_pairs_kernel<<<blocks(static_cast<long long>(V) + E), 128, 0, st>>>(t);
+    VBD_CUDA_TRY(cudaGetLastError());
+    table_entries_kernel<<<blocks(V), 128, 0, st>>>(t);
+    VBD_CUDA_TRY(cudaGetLastError());
+    return VBD_OK;
+}
+
+// the per-color passes are programmatic dependents of the kernel before them (each waits for it
+// with griddepcontrol.wait before its first read), so their launches overlap its tail
+template <typename... Args>
+static int launch_pass(void (*kernel)(Args...), int grid, int block, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    VBD_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, args...));
     return VBD_OK;
 }
 
@@ -1292,6 +1678,9 @@ int self_contact_accumulate(const VbdModelImpl& m, SelfContact& sc, const float4
     a.vbuf = sc.p.vertex_buffer;
     a.ebuf = sc.p.edge_buffer;
     a.tcap = sc.tcap;
+    a.ent_off = sc.ent_off;
+    a.ent = sc.ent;
+    a.ent_cap = sc.ent_cap;
     a.list = sc.act_v + m.color_start[color];
     a.count = sc.act_vcnt + color;
     a.r = sc.p.radius;
@@ -1307,12 +1696,11 @@ int self_contact_accumulate(const VbdModelImpl& m, SelfContact& sc, const float4
     // enough warps for every vertex of the color in one round, capped: the kernel strides
     const long long threads = static_cast<long long>(size) * kAccumLanes;
     const int grid = static_cast<int>(std::min<long long>((threads + 127) / 128, 148 * 16));
-    accumulate_kernel<<<grid, 128, 0, st>>>(a);
-    VBD_CUDA_TRY(cudaGetLastError());
-    return VBD_OK;
+    return launch_pass(accumulate_kernel, grid, 128, st, a);
 }
 
-int self_contact_truncate(const VbdModelImpl& m, SelfContact& sc, float4* pos, float4* disp, cudaStream_t st) {
+int self_contact_truncate(const VbdModelImpl& m, SelfContact& sc, float4* pos, float4* disp, int color,
+                          cudaStream_t st) {
     const int V = m.V;
     if (V == 0) return VBD_OK;
     TruncArgs a;
@@ -1324,6 +1712,11 @@ int self_contact_truncate(const VbdModelImpl& m, SelfContact& sc, float4* pos, f
     a.vt_list = sc.vt_list;
     a.ee_count = sc.ee_count;
     a.ee_list = sc.ee_list;
+    a.pair_off = sc.pair_off;
+    a.pair_ids = sc.pair_ids;
+    a.pair_n = sc.pair_n;
+    a.pair_h = sc.pair_h;
+    a.pair_cap = sc.pair_cap;
     a.V = V;
     a.E = m.E;
     a.vbuf = sc.p.vertex_buffer;
@@ -1331,14 +1724,12 @@ int self_contact_truncate(const VbdModelImpl& m, SelfContact& sc, float4* pos, f
     a.eps = sc.p.edge_parallel_epsilon;
     a.gamma = sc.p.relaxation;
     a.ts = sc.ts;
-    a.rows = sc.act_rows;
-    a.counts = sc.act_cnt;
-    const long long n = static_cast<long long>(std::max(V, m.E)) * kPlanarLanes;
-    planar_kernel<<<static_cast<int>(std::min<long long>((n + 127) / 128, 148 * 32)), 128, 0, st>>>(a);
-    VBD_CUDA_TRY(cudaGetLastError());
-    apply_truncation_kernel<<<(V + 255) / 256, 256, 0, st>>>(V, sc.cd, disp, pos, sc.ts, sc.max_disp);
-    VBD_CUDA_TRY(cudaGetLastError());
-    return VBD_OK;
+    // the number of pairs is on the device: about 16 per vertex before the grid strides
+    const long long n = 16LL * V;
+    const int rc = launch_pass(planar_kernel, static_cast<int>(std::min<long long>((n + 255) / 256, 148 * 8)), 256, st, a);
+    if (rc) return rc;
+    return launch_pass(apply_truncation_kernel, (V + 255) / 256, 256, st, V, const_cast<const float4*>(sc.cd), disp, pos,
+                       sc.ts, sc.max_disp, color < 0 ? 0 : m.color_start[color], color < 0 ? V : m.color_start[color + 1]);
 }
 
 }  // namespace vbd

@@ -74,14 +74,22 @@ struct SelfContact {
     int *ee_count = nullptr, *ee_list = nullptr;   // [E], [E * edge_buffer] edge ids ascending
     int *tv_count = nullptr, *tv_list = nullptr;   // [T], [T * tcap] internal vertex ids ascending
     // per-iteration state
-    unsigned char* flag = nullptr;  // [V] 1: the vertex takes part in a detected pair
     int C = 0;
     int* color_start = nullptr;  // [C+1] internal vertex ranges of the colors
     int* vcolor = nullptr;       // [V] color of each internal vertex (-1: none)
     int* act_v = nullptr;        // [V] contact-touching vertices, color c in [color_start[c], ...)
     int* act_vcnt = nullptr;     // [C] how many per color
-    int* act_rows = nullptr;     // [V + E] non-empty vertex-triangle rows, then non-empty edge rows
-    int* act_cnt = nullptr;      // [2] their counts
+    // per-vertex contact entries of the last detection (the force pass reads them in order): the
+    // four vertex ids of a pair, its kind and the vertex's slot in the ids' upper bits
+    long long *ent_cnt = nullptr, *ent_off = nullptr;  // [V+1]
+    int4* ent = nullptr;
+    long long ent_cap = 0;
+    // the detected pairs, flat (vertex-triangle rows, then edge-edge rows, each unordered pair once),
+    // with what the division plane needs of the base positions: unit normal and distance, heights
+    long long *pair_cnt = nullptr, *pair_off = nullptr;  // [V+E+1]
+    int4* pair_ids = nullptr;
+    float4 *pair_n = nullptr, *pair_h = nullptr;
+    long long pair_cap = 0;
     float4* cd = nullptr;    // pos_prev_collision_detection (internal order)
     float4* sc_f = nullptr;  // [V] self-contact force
     float4* sc_h0 = nullptr; // [V] Hessian xx xy xz yy
@@ -99,8 +107,10 @@ int self_contact_detect(const VbdModelImpl& m, SelfContact& sc, const float4* po
 // into sc_f / sc_h0 / sc_h1 (the other vertices hold zero since the last detection).
 int self_contact_accumulate(const VbdModelImpl& m, SelfContact& sc, const float4* pos, const float4* prev,
                             int color, float dt, float friction_epsilon, cudaStream_t st);
-// Planar truncation of all displacements, then pos := cd + disp for every vertex.
-int self_contact_truncate(const VbdModelImpl& m, SelfContact& sc, float4* pos, float4* disp, cudaStream_t st);
+// Planar truncation of all displacements, then pos := cd + disp for every vertex whose displacement
+// changed: those of `color` (-1: every vertex) and those that a plane shortens.
+int self_contact_truncate(const VbdModelImpl& m, SelfContact& sc, float4* pos, float4* disp, int color,
+                          cudaStream_t st);
 // Whether iteration `it` begins with a detection (particle_collision_detection_interval).
 bool self_contact_detect_now(const SelfContact& sc, int it);
 // Loads model-order positions [V,3] into cd (internal order) -- for detection from a given state.

@@ -171,10 +171,12 @@ __device__ __forceinline__ void add_slot(float b, float3 cf, float d2E, float3 n
 }
 
 // vertex p against triangle (a, b, c): adds the force / Hessian share of participant `slot`
-// (0, 1, 2 = a, b, c; 3 = p).  Returns false when the pair is not within the radius.
-__device__ __forceinline__ bool vt_contact_slot(float3 a, float3 b, float3 c, float3 p, float3 a0, float3 b0,
-                                                float3 c0, float3 p0, int slot, float r, float ke, float kd, float mu,
-                                                float eps_u, float dt, float3& f, Sym3& H) {
+// (0, 1, 2 = a, b, c; 3 = p).  start(k) loads participant k's step-start position, only for a pair
+// in contact.  Returns false when the pair is not within the radius.
+template <typename Start>
+__device__ __forceinline__ bool vt_contact_slot(float3 a, float3 b, float3 c, float3 p, Start start, int slot, float r,
+                                                float ke, float kd, float mu, float eps_u, float dt, float3& f,
+                                                Sym3& H) {
     float3 bary;
     const float3 cp = triangle_closest_point(a, b, c, p, bary);
     const float3 diff = p - cp;
@@ -184,8 +186,8 @@ __device__ __forceinline__ bool vt_contact_slot(float3 a, float3 b, float3 c, fl
     float dEdD, d2E;
     self_contact_norm(dis, r, ke, dEdD, d2E);
     const float3 cf = (-dEdD) * n;
-    const float3 cprev = bary.x * a0 + bary.y * b0 + bary.z * c0;
-    const float3 dx = (p - p0) - (cp - cprev);
+    const float3 cprev = bary.x * start(0) + bary.y * start(1) + bary.z * start(2);
+    const float3 dx = (p - start(3)) - (cp - cprev);
     float3 b1, b2;
     orthonormal_basis(n, b1, b2);
     float3 ff;
@@ -197,10 +199,12 @@ __device__ __forceinline__ bool vt_contact_slot(float3 a, float3 b, float3 c, fl
     return true;
 }
 
-// edge (e0, e1) against edge (g0, g1): adds the share of endpoint `slot` (0 = e0, 1 = e1)
-__device__ __forceinline__ bool ee_contact_slot(float3 e0, float3 e1, float3 g0, float3 g1, float3 e0a, float3 e1a,
-                                                float3 g0a, float3 g1a, int slot, float r, float ke, float kd, float mu,
-                                                float eps_u, float dt, float par_eps, float3& f, Sym3& H) {
+// edge (e0, e1) against edge (g0, g1): adds the share of endpoint `slot` (0 = e0, 1 = e1);
+// start(k) as above, participants e0, e1, g0, g1
+template <typename Start>
+__device__ __forceinline__ bool ee_contact_slot(float3 e0, float3 e1, float3 g0, float3 g1, Start start, int slot,
+                                                float r, float ke, float kd, float mu, float eps_u, float dt,
+                                                float par_eps, float3& f, Sym3& H) {
     float s, t, dis;
     closest_edge_edge(e0, e1, g0, g1, par_eps, s, t, dis);
     if (!(0.f < dis && dis < r)) return false;
@@ -210,7 +214,8 @@ __device__ __forceinline__ bool ee_contact_slot(float3 e0, float3 e1, float3 g0,
     float dEdD, d2E;
     self_contact_norm(dis, r, ke, dEdD, d2E);
     const float3 cf = (-dEdD) * n;
-    const float3 c1p = e0a + (e1a - e0a) * s, c2p = g0a + (g1a - g0a) * t;
+    const float3 e0a = start(0), g0a = start(2);
+    const float3 c1p = e0a + (start(1) - e0a) * s, c2p = g0a + (start(3) - g0a) * t;
     const float3 dx = (c1 - c1p) - (c2 - c2p);
     float3 b1, b2;
     orthonormal_basis(n, b1, b2);

@@ -1557,7 +1557,7 @@ static void enqueue_color(SolverImpl& s, int color, const VbdContacts* c, float 
     if (s.sc.on) {
         self_contact_accumulate(m, s.sc, s.pos, s.prev, color, dt, s.friction_epsilon, st);
         launch_sweep(a, s.lanes, m.any_tri_damping || m.any_edge_damping, false, s.block, st);
-        self_contact_truncate(m, s.sc, s.pos, s.disp, st);
+        self_contact_truncate(m, s.sc, s.pos, s.disp, color, st);
         return;
     }
     launch_sweep(a, s.lanes, damp, false, s.block, st, gate, smem);
@@ -1591,7 +1591,7 @@ static void enqueue_finalize(SolverImpl& s, float* q_in, float* q_out, float* qd
 // forward displacement (solver_vbd.py:2065-2100).
 static int self_contact_start(SolverImpl& s, cudaStream_t st) {
     int rc = self_contact_detect(*s.m, s.sc, s.prev, s.disp, false, st);
-    if (!rc) rc = self_contact_truncate(*s.m, s.sc, s.pos, s.disp, st);
+    if (!rc) rc = self_contact_truncate(*s.m, s.sc, s.pos, s.disp, -1, st);
     return rc;
 }
 
