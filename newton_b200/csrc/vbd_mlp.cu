@@ -4,15 +4,12 @@
 // to the inertia target (x_solved - y) from one-ring features; the Gauss-Seidel iterations then
 // start from y + prediction instead of y.  Every product accumulates in FP32 on the tensor cores.
 // Inference (vbd_mlp_forward; in the step mode also the features and the start, one launch) runs
-// on tcgen05.mma with FP16 operands and TMEM accumulators (vbd_mlp_tc.cuh).  Training is
-// hand-written too, on BF16 mma.sync m16n8k16 tiles with FP32 master weights:
-//   * mlp_tile_kernel: per warp, 16 samples through the three layers with the activations handed
-//     from one layer's accumulator fragments to the next layer's A fragments in registers; in
-//     training mode it continues with the backward pass (dY, dH2 = dY W3^T, dZ2, dH1 = dZ2 W2^T,
-//     dZ1) and stores the BF16 operands of the weight gradients;
-//   * gemm_tn_kernel: dW = A^T B over the sample dimension (split-K, FP32 partials), then a
-//     deterministic reduction; column sums give the bias gradients;
-//   * adam_kernel: Adam on FP32 master weights, refreshing the BF16 copies.
+// on tcgen05.mma with FP16 operands and TMEM accumulators (vbd_mlp_tc.cuh).  Training keeps FP32
+// master weights: vbd_mlp_train_tc.cuh computes loss and gradients in one pass on tcgen05.mma with
+// BF16 operands; adam_kernel updates the weights and refreshes the BF16 copies.  mlp_tile_kernel is
+// the mma.sync forward pass (vbd_mlp_forward_mma_sync): per warp, 16 samples through the three layers
+// with the activations handed from one layer's accumulator fragments to the next layer's A
+// fragments in registers.
 // Fragment layouts are those of the PTX ISA for mma.m16n8k16 (A row-major, B column-major):
 // lane = 4*g + t holds A rows g and g+8 at columns 2t, 2t+1 (+8), B column g at rows 2t, 2t+1
 // (+8), and C rows g and g+8 at columns 2t, 2t+1; ldmatrix (with .trans where the stored
@@ -27,6 +24,7 @@
 #include "vbd_internal.h"
 #include "vbd_math.cuh"
 #include "vbd_mlp_tc.cuh"
+#include "vbd_mlp_train_tc.cuh"
 
 namespace vbd {
 
@@ -56,9 +54,6 @@ __device__ __forceinline__ void ldsm_x4_t(unsigned (&r)[4], const void* p) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"(saddr(p)));
 }
-__device__ __forceinline__ void ldsm_x2(unsigned& r0, unsigned& r1, const void* p) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(saddr(p)));
-}
 __device__ __forceinline__ void ldsm_x2_t(unsigned& r0, unsigned& r1, const void* p) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(saddr(p)));
 }
@@ -73,39 +68,20 @@ __device__ __forceinline__ unsigned pack2(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<unsigned*>(&v);
 }
-__device__ __forceinline__ float2 unpack2(unsigned u) {
-    __nv_bfloat162 v = *reinterpret_cast<__nv_bfloat162*>(&u);
-    return __bfloat1622float2(v);
-}
 __device__ __forceinline__ float sigm(float z) { return 1.0f / (1.0f + __expf(-z)); }
 __device__ __forceinline__ float silu(float z) { return z * sigm(z); }
-__device__ __forceinline__ float dsilu(float z) {
-    const float s = sigm(z);
-    return s * (1.0f + z * (1.0f - s));
-}
 
 struct MlpArgs {
     int n;
     const float* params;     // FP32 blob (biases read from it)
     const uint16_t* w16;     // BF16 weight blob
     const float* X;          // [n][64]
-    float* Y;                // [n][3] or NULL
-    // training
-    const float* T;          // [n][3] targets or NULL (inference)
-    float grad_scale;        // dL/dY = grad_scale * 2 (y - t)
-    float* loss;             // sum of squared errors (monitoring; atomic)
-    __nv_bfloat16* Xb;       // [n][64]
-    __nv_bfloat16* H1;       // [n][128]
-    __nv_bfloat16* H2;       // [n][128]
-    __nv_bfloat16* dZ1;      // [n][128]
-    __nv_bfloat16* dZ2;      // [n][128]
-    __nv_bfloat16* dY;       // [n][8]
+    float* Y;                // [n][3]
 };
 
 constexpr size_t kTileSmem = (size_t)(kIn * kStrideH + kHid * kStrideH + kHid * kOutP + kWarps * 16 * kStrideX) * 2 +
                              (size_t)(kHid + kHid + kOutP) * 4;
 
-template <bool kTrain>
 __global__ void __launch_bounds__(kThreads) mlp_tile_kernel(MlpArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     __nv_bfloat16* sW1 = reinterpret_cast<__nv_bfloat16*>(smem);
@@ -148,14 +124,6 @@ __global__ void __launch_bounds__(kThreads) mlp_tile_kernel(MlpArgs a) {
             *reinterpret_cast<unsigned*>(myX + r * kStrideX + c) = pack2(v.x, v.y);
         }
         __syncwarp();
-        if (kTrain) {
-            for (int i = lane; i < 16 * kIn / 8; i += 32) {
-                const int r = i / (kIn / 8), c = (i % (kIn / 8)) * 8;
-                if (row0 + r < a.n)
-                    *reinterpret_cast<uint4*>(a.Xb + (size_t)(row0 + r) * kIn + c) =
-                        *reinterpret_cast<const uint4*>(myX + r * kStrideX + c);
-            }
-        }
         // ---- layer 1: Z1 = X W1 + b1 ----
         unsigned ax[4][4];
         for (int kt = 0; kt < 4; ++kt) ldsm_x4(ax[kt], myX + (lane & 15) * kStrideX + kt * 16 + (lane >> 4) * 8);
@@ -168,28 +136,13 @@ __global__ void __launch_bounds__(kThreads) mlp_tile_kernel(MlpArgs a) {
                 mma16816(acc[2 * np], ax[kt], b[0], b[1]);
                 mma16816(acc[2 * np + 1], ax[kt], b[2], b[3]);
             }
-        unsigned z1p[16][2];  // Z1 kept as bf16 pairs for the backward pass
         unsigned ah[8][4];    // H1 as A fragments of layer 2
         for (int nt = 0; nt < 16; ++nt) {
             const int c = nt * 8 + 2 * t4;
             const float z0 = acc[nt][0] + sB1[c], z1 = acc[nt][1] + sB1[c + 1];
             const float z2 = acc[nt][2] + sB1[c], z3 = acc[nt][3] + sB1[c + 1];
-            if (kTrain) {
-                z1p[nt][0] = pack2(z0, z1);
-                z1p[nt][1] = pack2(z2, z3);
-            }
             ah[nt >> 1][(nt & 1) * 2 + 0] = pack2(silu(z0), silu(z1));
             ah[nt >> 1][(nt & 1) * 2 + 1] = pack2(silu(z2), silu(z3));
-        }
-        if (kTrain) {
-            for (int nt = 0; nt < 16; ++nt) {
-                const int c = nt * 8 + 2 * t4;
-                if (row0 + g < a.n)
-                    *reinterpret_cast<unsigned*>(a.H1 + (size_t)(row0 + g) * kHid + c) = ah[nt >> 1][(nt & 1) * 2];
-                if (row0 + g + 8 < a.n)
-                    *reinterpret_cast<unsigned*>(a.H1 + (size_t)(row0 + g + 8) * kHid + c) =
-                        ah[nt >> 1][(nt & 1) * 2 + 1];
-            }
         }
         // ---- layer 2: Z2 = H1 W2 + b2 ----
         for (int nt = 0; nt < 16; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
@@ -202,29 +155,14 @@ __global__ void __launch_bounds__(kThreads) mlp_tile_kernel(MlpArgs a) {
                 mma16816(acc[2 * np + 1], a2, b[2], b[3]);
             }
         }
-        unsigned z2p[16][2];  // Z2 kept as bf16 pairs for the backward pass
         for (int nt = 0; nt < 16; ++nt) {
             const int c = nt * 8 + 2 * t4;
             acc[nt][0] += sB2[c];
             acc[nt][1] += sB2[c + 1];
             acc[nt][2] += sB2[c];
             acc[nt][3] += sB2[c + 1];
-            if (kTrain) {
-                z2p[nt][0] = pack2(acc[nt][0], acc[nt][1]);
-                z2p[nt][1] = pack2(acc[nt][2], acc[nt][3]);
-            }
             ah[nt >> 1][(nt & 1) * 2 + 0] = pack2(silu(acc[nt][0]), silu(acc[nt][1]));
             ah[nt >> 1][(nt & 1) * 2 + 1] = pack2(silu(acc[nt][2]), silu(acc[nt][3]));
-        }
-        if (kTrain) {
-            for (int nt = 0; nt < 16; ++nt) {
-                const int c = nt * 8 + 2 * t4;
-                if (row0 + g < a.n)
-                    *reinterpret_cast<unsigned*>(a.H2 + (size_t)(row0 + g) * kHid + c) = ah[nt >> 1][(nt & 1) * 2];
-                if (row0 + g + 8 < a.n)
-                    *reinterpret_cast<unsigned*>(a.H2 + (size_t)(row0 + g + 8) * kHid + c) =
-                        ah[nt >> 1][(nt & 1) * 2 + 1];
-            }
         }
         // ---- layer 3: Y = H2 W3 + b3 ----
         float y[4] = {0.f, 0.f, 0.f, 0.f};
@@ -239,146 +177,13 @@ __global__ void __launch_bounds__(kThreads) mlp_tile_kernel(MlpArgs a) {
         y[1] += sB3[c0 + 1];
         y[2] += sB3[c0];
         y[3] += sB3[c0 + 1];
-        if (a.Y) {
-            for (int h = 0; h < 2; ++h) {
-                const int r = row0 + g + 8 * h;
-                if (r >= a.n) continue;
-                if (c0 < kOut) a.Y[(size_t)r * kOut + c0] = y[2 * h];
-                if (c0 + 1 < kOut) a.Y[(size_t)r * kOut + c0 + 1] = y[2 * h + 1];
-            }
-        }
-        if (!kTrain) continue;
-        // ---- backward ----
-        float dy[4] = {0.f, 0.f, 0.f, 0.f};
-        float se = 0.f;
         for (int h = 0; h < 2; ++h) {
             const int r = row0 + g + 8 * h;
             if (r >= a.n) continue;
-            for (int q = 0; q < 2; ++q) {
-                const int c = c0 + q;
-                if (c >= kOut) continue;
-                const float e = y[2 * h + q] - a.T[(size_t)r * kOut + c];
-                se += e * e;
-                dy[2 * h + q] = a.grad_scale * 2.0f * e;
-            }
-        }
-        for (int off = 16; off > 0; off >>= 1) se += __shfl_xor_sync(0xffffffffu, se, off);
-        if (lane == 0 && a.loss) atomicAdd(a.loss, se);
-        if (row0 + g < a.n)
-            *reinterpret_cast<unsigned*>(a.dY + (size_t)(row0 + g) * kOutP + c0) = pack2(dy[0], dy[1]);
-        if (row0 + g + 8 < a.n)
-            *reinterpret_cast<unsigned*>(a.dY + (size_t)(row0 + g + 8) * kOutP + c0) = pack2(dy[2], dy[3]);
-        // dH2 = dY W3^T   (A = dY padded to K = 16; B[k][n] = W3[n][k])
-        const unsigned ady[4] = {pack2(dy[0], dy[1]), pack2(dy[2], dy[3]), 0u, 0u};
-        for (int nt = 0; nt < 16; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-        for (int np = 0; np < 8; ++np) {
-            unsigned b0, b1;  // matrices: rows n of tile 2np, rows n of tile 2np+1 (k 0..7)
-            ldsm_x2(b0, b1, sW3 + ((2 * np + (jj & 1)) * 8 + rr) * kOutP);
-            mma16816(acc[2 * np], ady, b0, 0u);
-            mma16816(acc[2 * np + 1], ady, b1, 0u);
-        }
-        unsigned adz2[8][4];
-        for (int nt = 0; nt < 16; ++nt) {
-            const int c = nt * 8 + 2 * t4;
-            const float2 za = unpack2(z2p[nt][0]), zb = unpack2(z2p[nt][1]);
-            const float d0 = acc[nt][0] * dsilu(za.x), d1 = acc[nt][1] * dsilu(za.y);
-            const float d2 = acc[nt][2] * dsilu(zb.x), d3 = acc[nt][3] * dsilu(zb.y);
-            adz2[nt >> 1][(nt & 1) * 2 + 0] = pack2(d0, d1);
-            adz2[nt >> 1][(nt & 1) * 2 + 1] = pack2(d2, d3);
-            if (row0 + g < a.n) *reinterpret_cast<unsigned*>(a.dZ2 + (size_t)(row0 + g) * kHid + c) = pack2(d0, d1);
-            if (row0 + g + 8 < a.n)
-                *reinterpret_cast<unsigned*>(a.dZ2 + (size_t)(row0 + g + 8) * kHid + c) = pack2(d2, d3);
-        }
-        // dH1 = dZ2 W2^T  (B[k][n] = W2[n][k]: plain ldmatrix on rows n)
-        for (int nt = 0; nt < 16; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-        for (int kt = 0; kt < 8; ++kt) {
-            const unsigned a2[4] = {adz2[kt][0], adz2[kt][1], adz2[kt][2], adz2[kt][3]};
-            for (int np = 0; np < 8; ++np) {
-                unsigned b[4];  // matrices: (tile 2np, k 0-7), (tile 2np, k 8-15), (tile 2np+1, k 0-7), (.., k 8-15)
-                ldsm_x4(b, sW2 + ((2 * np + (jj >> 1)) * 8 + rr) * kStrideH + kt * 16 + (jj & 1) * 8);
-                mma16816(acc[2 * np], a2, b[0], b[1]);
-                mma16816(acc[2 * np + 1], a2, b[2], b[3]);
-            }
-        }
-        for (int nt = 0; nt < 16; ++nt) {
-            const int c = nt * 8 + 2 * t4;
-            const float2 za = unpack2(z1p[nt][0]), zb = unpack2(z1p[nt][1]);
-            const float d0 = acc[nt][0] * dsilu(za.x), d1 = acc[nt][1] * dsilu(za.y);
-            const float d2 = acc[nt][2] * dsilu(zb.x), d3 = acc[nt][3] * dsilu(zb.y);
-            if (row0 + g < a.n) *reinterpret_cast<unsigned*>(a.dZ1 + (size_t)(row0 + g) * kHid + c) = pack2(d0, d1);
-            if (row0 + g + 8 < a.n)
-                *reinterpret_cast<unsigned*>(a.dZ1 + (size_t)(row0 + g + 8) * kHid + c) = pack2(d2, d3);
+            if (c0 < kOut) a.Y[(size_t)r * kOut + c0] = y[2 * h];
+            if (c0 + 1 < kOut) a.Y[(size_t)r * kOut + c0 + 1] = y[2 * h + 1];
         }
     }
-}
-
-// dW[M][N] = sum_s A[s][m] * B[s][n] for s in this split's sample range (FP32 partials).
-constexpr int kGemmK = 32;
-__global__ void __launch_bounds__(128) gemm_tn_kernel(int S, const __nv_bfloat16* A, int M, const __nv_bfloat16* B,
-                                                       int N, int samples_per_split, float* part) {
-    __shared__ __align__(16) __nv_bfloat16 sA[kGemmK][64 + 8];
-    __shared__ __align__(16) __nv_bfloat16 sB[kGemmK][64 + 8];
-    const int m0 = blockIdx.x * 64, n0 = blockIdx.y * 64, split = blockIdx.z;
-    const int s_begin = split * samples_per_split, s_end = min(S, s_begin + samples_per_split);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int g = lane >> 2, t4 = lane & 3, jj = lane >> 3, rr = lane & 7;
-    const int nN = min(64, N - n0);
-    float acc[8][4];
-    for (int i = 0; i < 8; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-    for (int s0 = s_begin; s0 < s_end; s0 += kGemmK) {
-        for (int i = tid; i < kGemmK * 8; i += 128) {  // 32 rows x 8 chunks of 8 bf16
-            const int r = i >> 3, c = (i & 7) * 8;
-            const int s = s0 + r;
-            uint4 va = make_uint4(0, 0, 0, 0), vb = make_uint4(0, 0, 0, 0);
-            if (s < s_end) {
-                va = *reinterpret_cast<const uint4*>(A + (size_t)s * M + m0 + c);
-                if (c < nN) vb = *reinterpret_cast<const uint4*>(B + (size_t)s * N + n0 + c);
-            }
-            *reinterpret_cast<uint4*>(&sA[r][c]) = va;
-            *reinterpret_cast<uint4*>(&sB[r][c]) = vb;
-        }
-        __syncthreads();
-        for (int kt = 0; kt < kGemmK / 16; ++kt) {
-            unsigned af[4];
-            ldsm_x4_t(af, &sA[kt * 16 + (jj >> 1) * 8 + rr][warp * 16 + (jj & 1) * 8]);
-            for (int np = 0; np < 4; ++np) {
-                unsigned b[4];
-                ldsm_x4_t(b, &sB[kt * 16 + (jj & 1) * 8 + rr][(2 * np + (jj >> 1)) * 8]);
-                mma16816(acc[2 * np], af, b[0], b[1]);
-                mma16816(acc[2 * np + 1], af, b[2], b[3]);
-            }
-        }
-        __syncthreads();
-    }
-    float* out = part + (size_t)split * M * N;
-    for (int nt = 0; nt < 8; ++nt) {
-        const int n = n0 + nt * 8 + 2 * t4;
-        if (nt * 8 >= nN) continue;
-        const int m = m0 + warp * 16 + g;
-        out[(size_t)m * N + n] = acc[nt][0];
-        out[(size_t)m * N + n + 1] = acc[nt][1];
-        out[(size_t)(m + 8) * N + n] = acc[nt][2];
-        out[(size_t)(m + 8) * N + n + 1] = acc[nt][3];
-    }
-}
-
-// out[i] = sum over splits, in split order (deterministic).
-__global__ void reduce_splits_kernel(const float* part, int splits, int count, float* out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    float s = 0.f;
-    for (int k = 0; k < splits; ++k) s += part[(size_t)k * count + i];
-    out[i] = s;
-}
-
-// column sums of a bf16 [S][C] matrix: per-block partials over row chunks, then reduce_splits
-__global__ void colsum_kernel(int S, const __nv_bfloat16* D, int C, int rows_per_block, float* part) {
-    const int c = threadIdx.x;
-    if (c >= C) return;
-    const int r0 = blockIdx.x * rows_per_block, r1 = min(S, r0 + rows_per_block);
-    float s = 0.f;
-    for (int r = r0; r < r1; ++r) s += __bfloat162float(D[(size_t)r * C + c]);
-    part[(size_t)blockIdx.x * C + c] = s;
 }
 
 __global__ void adam_kernel(float* p, const float* gr, float* m1, float* m2, uint16_t* w16, int n, float lr, float b1,
@@ -427,10 +232,10 @@ int ensure_tile_smem() {
     if (dev < 0 || dev >= 64) return fail(VBD_ERR_UNSUPPORTED, "vbd_mlp: device ordinal too large");
     std::lock_guard<std::mutex> lock(g_attr_mutex);
     if (!g_attr_done[dev]) {
-        VBD_CUDA_TRY(cudaFuncSetAttribute(mlp_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        VBD_CUDA_TRY(cudaFuncSetAttribute(mlp_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           static_cast<int>(kTileSmem)));
-        VBD_CUDA_TRY(cudaFuncSetAttribute(mlp_tile_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          static_cast<int>(kTileSmem)));
+        VBD_CUDA_TRY(cudaFuncSetAttribute(tct::mlp_train_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          tct::kSmemBytes));
         VBD_CUDA_TRY(cudaFuncSetAttribute(tc::mlp_infer_tc_kernel<tc::kInF32>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSmemBytes));
         VBD_CUDA_TRY(cudaFuncSetAttribute(tc::mlp_infer_tc_kernel<tc::kInStep>,
@@ -664,15 +469,15 @@ extern "C" int vbd_mlp_sizes(int32_t* params, int32_t* weights16, int32_t* in_fe
     return VBD_OK;
 }
 
+namespace vbd {
+// CTAs of the training kernel: one per 128-sample tile, at most one per SM of a B200
+static int train_ctas(int n) { return std::min(tct::kMaxCtas, (n + tct::kRows - 1) / tct::kRows); }
+}  // namespace vbd
+
 extern "C" int vbd_mlp_workspace_bytes(int32_t n, int64_t* bytes) {
     if (n < 0 || !bytes) return fail(VBD_ERR_INVALID_ARGUMENT, "vbd_mlp_workspace_bytes: bad arguments");
-    const size_t rows = static_cast<size_t>(n);
-    const int splits = 64;
-    size_t b = rows * (kIn + 4 * kHid + kOutP) * 2;               // bf16 operands
-    b = (b + 255) & ~static_cast<size_t>(255);
-    b += static_cast<size_t>(splits) * kHid * kHid * 4;           // GEMM partials (largest)
-    b += static_cast<size_t>(1024) * kHid * 4;                    // column-sum partials
-    *bytes = static_cast<int64_t>(b);
+    // one partial of the parameter gradients per CTA of the training kernel
+    *bytes = static_cast<int64_t>(std::max(train_ctas(n), 1)) * tct::kPart * 4;
     return VBD_OK;
 }
 
@@ -772,7 +577,7 @@ extern "C" int vbd_mlp_forward_mma_sync(const float* params, const uint16_t* w16
     a.w16 = w16;
     a.X = X;
     a.Y = Y;
-    mlp_tile_kernel<false><<<tile_grid(n), kThreads, kTileSmem, static_cast<cudaStream_t>(stream)>>>(a);
+    mlp_tile_kernel<<<tile_grid(n), kThreads, kTileSmem, static_cast<cudaStream_t>(stream)>>>(a);
     VBD_CUDA_TRY(cudaGetLastError());
     return VBD_OK;
 }
@@ -798,9 +603,7 @@ extern "C" int vbd_mlp_backward(const float* params, const uint16_t* w16, const 
     int rc = ensure_tile_smem();
     if (rc) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const size_t rows = static_cast<size_t>(n);
-    __nv_bfloat16* base = static_cast<__nv_bfloat16*>(workspace);
-    MlpArgs a;
+    tct::TrainArgs a;
     std::memset(&a, 0, sizeof(a));
     a.n = n;
     a.params = params;
@@ -808,42 +611,17 @@ extern "C" int vbd_mlp_backward(const float* params, const uint16_t* w16, const 
     a.X = X;
     a.T = T;
     a.grad_scale = grad_scale;
-    a.loss = loss;
-    a.Xb = base;
-    a.H1 = a.Xb + rows * kIn;
-    a.H2 = a.H1 + rows * kHid;
-    a.dZ1 = a.H2 + rows * kHid;
-    a.dZ2 = a.dZ1 + rows * kHid;
-    a.dY = a.dZ2 + rows * kHid;
-    size_t off = rows * (kIn + 4 * kHid + kOutP) * 2;
-    off = (off + 255) & ~static_cast<size_t>(255);
-    float* part = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + off);
-    float* cpart = part + static_cast<size_t>(64) * kHid * kHid;
-    mlp_tile_kernel<true><<<tile_grid(n), kThreads, kTileSmem, st>>>(a);
+    a.part = static_cast<float*>(workspace);
+    unsigned* counter = nullptr;
+    VBD_CUDA_TRY(cudaGetSymbolAddress(reinterpret_cast<void**>(&counter), g_mlp_tc_timeouts));
+    a.status = counter;
+    const int ctas = train_ctas(n);
+    tct::mlp_train_tc_kernel<<<ctas, tct::kThreads, tct::kSmemBytes, st>>>(a);
     VBD_CUDA_TRY(cudaGetLastError());
-    const int splits = std::min(64, (n + 511) / 512);
-    const int per_split = ((n + splits - 1) / splits + kGemmK - 1) / kGemmK * kGemmK;
-    auto dW = [&](const __nv_bfloat16* Am, int M, const __nv_bfloat16* Bm, int N, float* out) -> int {
-        dim3 grid(M / 64, (N + 63) / 64, splits);
-        gemm_tn_kernel<<<grid, 128, 0, st>>>(n, Am, M, Bm, N, per_split, part);
-        reduce_splits_kernel<<<(M * N + 255) / 256, 256, 0, st>>>(part, splits, M * N, out);
-        VBD_CUDA_TRY(cudaGetLastError());
-        return VBD_OK;
-    };
-    auto db = [&](const __nv_bfloat16* D, int C, float* out) -> int {
-        const int blocks = std::min(1024, (n + 255) / 256);
-        const int rpb = (n + blocks - 1) / blocks;
-        colsum_kernel<<<blocks, 128, 0, st>>>(n, D, C, rpb, cpart);
-        reduce_splits_kernel<<<(C + 255) / 256, 256, 0, st>>>(cpart, blocks, C, out);
-        VBD_CUDA_TRY(cudaGetLastError());
-        return VBD_OK;
-    };
-    if ((rc = dW(a.Xb, kIn, a.dZ1, kHid, grads + kOffW1))) return rc;
-    if ((rc = db(a.dZ1, kHid, grads + kOffB1))) return rc;
-    if ((rc = dW(a.H1, kHid, a.dZ2, kHid, grads + kOffW2))) return rc;
-    if ((rc = db(a.dZ2, kHid, grads + kOffB2))) return rc;
-    if ((rc = dW(a.H2, kHid, a.dY, kOutP, grads + kOffW3))) return rc;
-    if ((rc = db(a.dY, kOutP, grads + kOffB3))) return rc;
+    const int cols = tct::kParams + 1;  // and the loss
+    tct::mlp_train_reduce_kernel<<<(cols + tct::kReduceWidth - 1) / tct::kReduceWidth,
+                                   tct::kReduceWidth * tct::kReduceChains, 0, st>>>(a.part, ctas, grads, loss);
+    VBD_CUDA_TRY(cudaGetLastError());
     return VBD_OK;
 }
 
