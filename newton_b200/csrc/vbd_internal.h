@@ -80,7 +80,8 @@ struct VbdModelImpl {
     float4* tri_D = nullptr;          // [n_tri_rec] DmInv 00, 01, 10, 11
     float4* tri_mat = nullptr;        // [n_tri_rec] area, mu, lambda, kd
     int4* edge_idx = nullptr;         // [n_edge_rec] o0, o1, v0, v1 (internal ids); order in bits 30-31 of .x
-    float4* edge_mat = nullptr;       // [n_edge_rec] rest angle, rest length, ke, kd
+    float2* edge_mat = nullptr;       // [n_edge_rec] rest angle, ke * rest length
+    float* edge_kd = nullptr;         // [n_edge_rec] kd * rest length (NULL: no bending damping)
     DevShape* shapes = nullptr;       // [S]
     int n_worlds = 0;                 // W: 1 + the largest particle or shape world id
     int* world_shape_offsets = nullptr;   // [W+2] CSR rows: world w -> its shapes and the global ones
@@ -95,7 +96,7 @@ struct VbdModelImpl {
     // host copies of the layout (used to build the shared-memory-resident patches)
     std::vector<float4> pinfo_h;
     std::vector<int4> vadj_h, tri_idx_h, edge_idx_h;
-    std::vector<float4> tri_D_h, tri_mat_h, edge_mat_h;
+    std::vector<float4> tri_D_h, tri_mat_h, edge_mat_h;  // (edge_mat_h: rest angle, rest length, ke, kd)
     std::vector<int> tri_elem_h, edge_elem_h;   // element id of each record (dedupe per patch)
     std::vector<float> rest_q_h;                // [3V] initial positions in internal order (may be empty)
     // raw topology in model order (self-contact layer) and the model-level contact material

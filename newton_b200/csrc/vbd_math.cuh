@@ -71,15 +71,29 @@ __device__ __forceinline__ Sym3 zero_sym() { Sym3 h = {0.f, 0.f, 0.f, 0.f, 0.f, 
 // `* area` (particle_vbd_kernels.py:629-630) into the moduli is the same expression.
 // Restates particle_vbd_kernels.py:502-632 otherwise term by term.
 // ---------------------------------------------------------------------------------------------
-template <bool kDamping>
-__device__ __forceinline__ void membrane_eval(int order, float3 x0, float3 x1, float3 x2, float3 a0,
-                                              float3 a1, float3 a2, float4 D, float4 mat, float inv_dt,
-                                              float3& f, Sym3& h) {
-    const float mu = mat.x, lnh = mat.y, alpha = mat.z, kd = mat.w;
+// F of the triangle and the products the energy needs
+__device__ __forceinline__ void membrane_F(float3 x0, float3 x1, float3 x2, float4 D, float3& F0, float3& F1) {
     const float3 x01 = x1 - x0;
     const float3 x02 = x2 - x0;
-    const float3 F0 = x01 * D.x + x02 * D.z;
-    const float3 F1 = x01 * D.y + x02 * D.w;
+    F0 = x01 * D.x + x02 * D.z;
+    F1 = x01 * D.y + x02 * D.w;
+}
+
+// F^T F = (F0.F0, F0.F1, F1.F1) of the triangle at the step's start, for damping: the same for all
+// sweeps of a step, so it is computed once per step
+__device__ __forceinline__ float3 membrane_metric(float3 a0, float3 a1, float3 a2, float4 D) {
+    float3 F0, F1;
+    membrane_F(a0, a1, a2, D, F0, F1);
+    return f3(dot(F0, F0), dot(F0, F1), dot(F1, F1));
+}
+
+// c_prev: membrane_metric (read only with damping)
+template <bool kDamping>
+__device__ __forceinline__ void membrane_eval(int order, float3 x0, float3 x1, float3 x2, float3 c_prev, float4 D,
+                                              float4 mat, float inv_dt, float3& f, Sym3& h) {
+    const float mu = mat.x, lnh = mat.y, alpha = mat.z, kd = mat.w;
+    float3 F0, F1;
+    membrane_F(x0, x1, x2, D, F0, F1);
     const float c00 = dot(F0, F0), c11 = dot(F1, F1), c01 = dot(F0, F1);
     const float js2 = fmaxf(c00 * c11 - c01 * c01, 1.0e-20f);
     const float inv_js = rsqrtf(js2);
@@ -94,23 +108,27 @@ __device__ __forceinline__ void membrane_eval(int order, float3 x0, float3 x1, f
     const float d1 = order == 0 ? -(D.y + D.w) : (order == 1 ? D.y : D.w);
     f = f - (P0 * d0 + P1 * d1);
 
-    const float r = fmaxf(0.0f, s) * inv_js;
-    const float cJ = lnh - r;
     const float3 dJ = g0 * d0 + g1 * d1;
-    const float3 w = F1 * d0 - F0 * d1;
-    const float icoef = mu * (d0 * d0 + d1 * d1) + r * (d0 * d0 * c11 + d1 * d1 * c00 - 2.0f * d0 * d1 * c01);
-    add_diag(h, icoef);
-    add_outer(h, cJ, dJ);
-    add_outer(h, -r, w);
+    const float dd = d0 * d0 + d1 * d1;
+    if (s > 0.0f) {
+        // the clamped second-derivative terms: zero unless the area has grown beyond alpha, which
+        // cloth rarely does, so whole warps skip about 25 instructions.  (With r = 0 they would add
+        // zeros: both branches give the bits of the one formula.)
+        const float r = s * inv_js;
+        const float3 w = F1 * d0 - F0 * d1;
+        const float icoef = mu * dd + r * (d0 * d0 * c11 + d1 * d1 * c00 - 2.0f * d0 * d1 * c01);
+        add_diag(h, icoef);
+        add_outer(h, lnh - r, dJ);
+        add_outer(h, -r, w);
+    } else {
+        add_diag(h, __fmul_rn(mu, dd));
+        add_outer(h, lnh, dJ);
+    }
 
     if (kDamping && kd > 0.0f) {
-        const float3 p01 = a1 - a0;
-        const float3 p02 = a2 - a0;
-        const float3 F0p = p01 * D.x + p02 * D.z;
-        const float3 F1p = p01 * D.y + p02 * D.w;
-        const float r00 = (c00 - dot(F0p, F0p)) * inv_dt;
-        const float r01 = (c01 - dot(F0p, F1p)) * inv_dt;
-        const float r11 = (c11 - dot(F1p, F1p)) * inv_dt;
+        const float r00 = (c00 - c_prev.x) * inv_dt;
+        const float r01 = (c01 - c_prev.y) * inv_dt;
+        const float r11 = (c11 - c_prev.z) * inv_dt;
         const float3 e00 = (2.0f * d0) * F0;
         const float3 e01 = d0 * F1 + d1 * F0;
         const float3 e11 = (2.0f * d1) * F1;
@@ -149,100 +167,88 @@ __device__ __forceinline__ float atan2_as(float y, float x) {
 
 // ---------------------------------------------------------------------------------------------
 // Dihedral-angle bending of one hinge (o0, o1, v0, v1) = (x0, x1, x2, x3); `order` selects the
-// vertex.  em = (rest_angle, rest_length, ke, kd).  Restates particle_vbd_kernels.py:664-816.
+// vertex.  k, kd = ke, kd times the rest length.  Restates particle_vbd_kernels.py:664-816.
 // The caller has already dropped boundary hinges (o0 or o1 == -1, which the reference returns
 // as exact zero) and hinges with ke <= 0 (which the reference never evaluates).
 // ---------------------------------------------------------------------------------------------
+constexpr float kNoAngle = 1.0e30f;  // step-start angle of a degenerate hinge: no damping
+
 __device__ __forceinline__ float3 project_cross(float inv_len, float3 nh, float3 y, float3 u) {
     // (1/|n|) (I - nh nh^T) y  x  u
     const float3 p = (y - nh * dot(nh, y)) * inv_len;
     return cross(p, u);
 }
 
-// kSelect: form both projections for every order and select the result afterwards (straight-line
-// code, so that the caller can interleave the evaluation of independent hinges); otherwise branch
-// on the order (fewer live registers).  Both compute the same operations for a given order, so
-// they give the same bits.
-template <bool kDamping, bool kSelect = false>
-__device__ __forceinline__ void bending_eval(int order, float3 x0, float3 x1, float3 x2, float3 x3, float3 a0,
-                                             float3 a1, float3 a2, float3 a3, float4 em, float inv_dt, float3& f,
-                                             Sym3& h) {
+// unit normals n1h, n2h, unit hinge eh, their inverse lengths, and the angle; false: degenerate
+struct Hinge {
+    float3 n1h, n2h, eh;
+    float i1, i2, sin_t, cos_t, theta;
+};
+
+__device__ __forceinline__ bool hinge_set(float3 x02, float3 x03, float3 x13, float3 x12, float3 e, Hinge& g) {
     const float eps = 1.0e-6f;
+    const float3 n1 = cross(x02, x03);
+    const float3 n2 = cross(x13, x12);
+    // |n| < eps  <=>  |n|^2 < eps^2; the unit vectors use the hardware reciprocal square root
+    const float d1 = dot(n1, n1), d2 = dot(n2, n2), de = dot(e, e);
+    if (d1 < eps * eps || d2 < eps * eps || de < eps * eps) return false;
+    g.i1 = rsqrtf(d1);
+    g.i2 = rsqrtf(d2);
+    g.n1h = n1 * g.i1;
+    g.n2h = n2 * g.i2;
+    g.eh = e * rsqrtf(de);
+    g.sin_t = dot(cross(g.n1h, g.n2h), g.eh);
+    g.cos_t = dot(g.n1h, g.n2h);
+    g.theta = atan2_as(g.sin_t, g.cos_t);
+    return true;
+}
+
+// the hinge's angle at the step's start (kNoAngle: degenerate), for damping: once per step
+__device__ __forceinline__ float hinge_angle(float3 a0, float3 a1, float3 a2, float3 a3) {
+    Hinge g;
+    return hinge_set(a2 - a0, a3 - a0, a3 - a1, a2 - a1, a3 - a2, g) ? g.theta : kNoAngle;
+}
+
+// Both projections are formed for every order and the result selected afterwards: a warp holds
+// hinges of all four orders, so that branches on the order would run one after the other (the two
+// forms compute the same operations for a given order and give the same bits).  With the damping tables
+// and the area branch, a warp of 8 vertices takes 1,402 instructions per sweep instead of 1,694.
+template <bool kDamping>
+__device__ __forceinline__ void bending_eval(int order, float3 x0, float3 x1, float3 x2, float3 x3, float theta_prev,
+                                             float rest, float k, float kd, float inv_dt, float3& f, Sym3& h) {
     const float3 x02 = x2 - x0;
     const float3 x03 = x3 - x0;
     const float3 x13 = x3 - x1;
     const float3 x12 = x2 - x1;
     const float3 e = x3 - x2;
-    const float3 n1 = cross(x02, x03);
-    const float3 n2 = cross(x13, x12);
-    // |n| < eps  <=>  |n|^2 < eps^2; the unit vectors use the hardware reciprocal square root
-    const float d1 = dot(n1, n1), d2 = dot(n2, n2), de = dot(e, e);
-    if (d1 < eps * eps || d2 < eps * eps || de < eps * eps) return;
-    const float i1 = rsqrtf(d1), i2 = rsqrtf(d2), ie = rsqrtf(de);
-    const float3 n1h = n1 * i1;
-    const float3 n2h = n2 * i2;
-    const float3 eh = e * ie;
-    const float sin_t = dot(cross(n1h, n2h), eh);
-    const float cos_t = dot(n1h, n2h);
-    const float theta = atan2_as(sin_t, cos_t);
-    const float k = em.z * em.y;
-    const float dE = k * (theta - em.x);
+    Hinge q;
+    if (!hinge_set(x02, x03, x13, x12, e, q)) return;
+    const float dE = k * (q.theta - rest);
 
-    // Selected dtheta/dx (see header comment).
-    float3 g;
-    if (kSelect) {
-        //   order 0:  T1(y1) x e            order 2:  T2(y2) x x13 - T1(y1) x x03
-        //   order 1: -T2(y2) x e            order 3:  T1(y1) x x02 - T2(y2) x x12
-        const float3 y1 = -cos_t * cross(eh, n2h) - sin_t * n2h;
-        const float3 y2 = cos_t * cross(eh, n1h) - sin_t * n1h;
-        const float3 u1 = order == 0 ? e : (order == 2 ? x03 : x02);
-        const float3 u2 = order == 1 ? e : (order == 2 ? x13 : x12);
-        const float3 t1 = project_cross(i1, n1h, y1, u1);
-        const float3 t2 = project_cross(i2, n2h, y2, u2);
-        const float3 d12 = t1 - t2;
-        g = order == 0 ? t1 : (order == 1 ? -t2 : (order == 2 ? -d12 : d12));
-    } else if (order == 0) {
-        const float3 y1 = -cos_t * cross(eh, n2h) - sin_t * n2h;
-        g = project_cross(i1, n1h, y1, e);
-    } else if (order == 1) {
-        const float3 y2 = cos_t * cross(eh, n1h) - sin_t * n1h;
-        g = -project_cross(i2, n2h, y2, e);
-    } else if (order == 2) {
-        const float3 y1 = -cos_t * cross(eh, n2h) - sin_t * n2h;
-        const float3 y2 = cos_t * cross(eh, n1h) - sin_t * n1h;
-        g = project_cross(i2, n2h, y2, x13) - project_cross(i1, n1h, y1, x03);
-    } else {
-        const float3 y1 = -cos_t * cross(eh, n2h) - sin_t * n2h;
-        const float3 y2 = cos_t * cross(eh, n1h) - sin_t * n1h;
-        g = project_cross(i1, n1h, y1, x02) - project_cross(i2, n2h, y2, x12);
-    }
+    // Selected dtheta/dx (see header comment):
+    //   order 0:  T1(y1) x e            order 2:  T2(y2) x x13 - T1(y1) x x03
+    //   order 1: -T2(y2) x e            order 3:  T1(y1) x x02 - T2(y2) x x12
+    const float3 y1 = -q.cos_t * cross(q.eh, q.n2h) - q.sin_t * q.n2h;
+    const float3 y2 = q.cos_t * cross(q.eh, q.n1h) - q.sin_t * q.n1h;
+    const float3 u1 = order == 0 ? e : (order == 2 ? x03 : x02);
+    const float3 u2 = order == 1 ? e : (order == 2 ? x13 : x12);
+    const float3 t1 = project_cross(q.i1, q.n1h, y1, u1);
+    const float3 t2 = project_cross(q.i2, q.n2h, y2, u2);
+    const float3 d12 = t1 - t2;
+    const float3 g = order == 0 ? t1 : (order == 1 ? -t2 : (order == 2 ? -d12 : d12));
     f = f + (-dE) * g;
     add_outer(h, k, g);
 
-    if (kDamping && em.w > 0.0f) {
-        const float3 p02 = a2 - a0;
-        const float3 p03 = a3 - a0;
-        const float3 p13 = a3 - a1;
-        const float3 p12 = a2 - a1;
-        const float3 pe = a3 - a2;
-        const float3 q1 = cross(p02, p03);
-        const float3 q2 = cross(p13, p12);
-        const float s1 = dot(q1, q1), s2 = dot(q2, q2), se = dot(pe, pe);
-        if (s1 < eps * eps || s2 < eps * eps || se < eps * eps) return;
-        const float3 q1h = q1 * rsqrtf(s1);
-        const float3 q2h = q2 * rsqrtf(s2);
-        const float3 qeh = pe * rsqrtf(se);
-        const float theta_prev = atan2_as(dot(cross(q1h, q2h), qeh), dot(q1h, q2h));
-        float dth = theta - theta_prev;
+    if (kDamping && kd > 0.0f && theta_prev != kNoAngle) {
+        float dth = q.theta - theta_prev;
         if (dth > 3.141592653589793f) {
             dth = dth - 6.283185307179586f;
         } else if (dth < -3.141592653589793f) {
             dth = dth + 6.283185307179586f;
         }
         const float rate = dth * inv_dt;
-        const float kdl = em.w * em.y;
-        f = f + (-kdl * rate) * g;
-        add_outer(h, kdl * inv_dt, g);
+        f = f + (-kd * rate) * g;
+        add_outer(h, kd * inv_dt, g);
     }
 }
 

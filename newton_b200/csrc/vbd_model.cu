@@ -40,7 +40,7 @@ static int upload(T** dst, const std::vector<T>& src) {
 static void free_model(VbdModelImpl& m) {
     void* ptrs[] = {m.perm,       m.inv_perm, m.pinfo,          m.vadj,
                     m.tri_idx,    m.tri_D,    m.tri_mat,        m.edge_idx,
-                    m.edge_mat,   m.shapes,   m.particle_world, m.particle_flags_orig,
+                    m.edge_mat,   m.edge_kd,  m.shapes,   m.particle_world, m.particle_flags_orig,
                     m.particle_radius_orig, m.nbr8, m.vfeat, m.world_shape_offsets, m.world_shapes};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -51,6 +51,7 @@ static void free_model(VbdModelImpl& m) {
     m.tri_D = m.tri_mat = nullptr;
     m.edge_idx = nullptr;
     m.edge_mat = nullptr;
+    m.edge_kd = nullptr;
     m.shapes = nullptr;
     m.particle_world = m.particle_flags_orig = nullptr;
     m.particle_radius_orig = nullptr;
@@ -209,6 +210,8 @@ static int build_model(const VbdModelDesc* d, VbdModelImpl& m) {
     std::vector<float4> tri_D(n_tri_rec), tri_mat(n_tri_rec);
     std::vector<int4> edge_idx(n_edge_rec);
     std::vector<float4> edge_mat(n_edge_rec);
+    std::vector<float2> edge_rk(n_edge_rec);
+    std::vector<float> edge_kd(n_edge_rec);
     m.tri_elem_h.assign(n_tri_rec, 0);
     m.edge_elem_h.assign(n_edge_rec, 0);
     std::atomic<bool> any_tri_damp{false}, any_edge_damp{false};
@@ -252,7 +255,10 @@ static int build_model(const VbdModelDesc* d, VbdModelImpl& m) {
                     const float ke = d->edge_bending_properties[2 * ed], kd = d->edge_bending_properties[2 * ed + 1];
                     edge_idx[r] = make_int4(inv[ei[0]] | (slot << 30), inv[ei[1]], inv[ei[2]], inv[ei[3]]);
                     m.edge_elem_h[r] = ed;
-                    edge_mat[r] = make_float4(d->edge_rest_angle[ed], d->edge_rest_length[ed], ke, kd);
+                    const float rest = d->edge_rest_angle[ed], len = d->edge_rest_length[ed];
+                    edge_mat[r] = make_float4(rest, len, ke, kd);
+                    edge_rk[r] = make_float2(rest, ke * len);
+                    edge_kd[r] = kd * len;
                     edamp |= kd > 0.0f;
                     ++r;
                 }
@@ -362,7 +368,8 @@ static int build_model(const VbdModelDesc* d, VbdModelImpl& m) {
     if ((rc = upload(&m.tri_D, tri_D))) return rc;
     if ((rc = upload(&m.tri_mat, tri_mat))) return rc;
     if ((rc = upload(&m.edge_idx, edge_idx))) return rc;
-    if ((rc = upload(&m.edge_mat, edge_mat))) return rc;
+    if ((rc = upload(&m.edge_mat, edge_rk))) return rc;
+    if (m.any_edge_damping && (rc = upload(&m.edge_kd, edge_kd))) return rc;
     if ((rc = upload(&m.shapes, m.shapes_host))) return rc;
     if ((rc = upload(&m.particle_world, pworld))) return rc;
     if ((rc = upload(&m.particle_flags_orig, pflags))) return rc;

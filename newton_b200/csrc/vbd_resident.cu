@@ -206,14 +206,11 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(ResidentK
                     const ushort4 ti = s_tri_idx[e];
                     const float4 mt = s_tri_mat[e];
                     const float3 x0 = xyz(s_pos[ti.x]), x1 = xyz(s_pos[ti.y]), x2 = xyz(s_pos[ti.z]);
-                    float3 p0 = x0, p1 = x1, p2 = x2;
-                    if (kDamp && mt.w > 0.0f) {
-                        p0 = xyz(s_prev[ti.x]);
-                        p1 = xyz(s_prev[ti.y]);
-                        p2 = xyz(s_prev[ti.z]);
-                    }
-                    membrane_eval<kDamp>(static_cast<int>(ref & 3u), x0, x1, x2, p0, p1, p2, s_tri_D[e], mt, inv_dt,
-                                         f, h);
+                    const float4 D = s_tri_D[e];
+                    float3 c = f3(0.f, 0.f, 0.f);
+                    if (kDamp && mt.w > 0.0f)
+                        c = membrane_metric(xyz(s_prev[ti.x]), xyz(s_prev[ti.y]), xyz(s_prev[ti.z]), D);
+                    membrane_eval<kDamp>(static_cast<int>(ref & 3u), x0, x1, x2, c, D, mt, inv_dt, f, h);
                 }
                 // hinges continue the round-robin deal of the merged record list
                 const int lane_e = (lane - (vr.y - vr.x) % kLanes + kLanes) % kLanes;
@@ -224,14 +221,11 @@ __global__ void __launch_bounds__(kResidentThreads, 1) resident_kernel(ResidentK
                     const float4 em = s_hinge_mat[e];
                     const float3 x0 = xyz(s_pos[hi.x]), x1 = xyz(s_pos[hi.y]), x2 = xyz(s_pos[hi.z]),
                                  x3 = xyz(s_pos[hi.w]);
-                    float3 p0 = x0, p1 = x1, p2 = x2, p3 = x3;
-                    if (kDamp && em.w > 0.0f) {
-                        p0 = xyz(s_prev[hi.x]);
-                        p1 = xyz(s_prev[hi.y]);
-                        p2 = xyz(s_prev[hi.z]);
-                        p3 = xyz(s_prev[hi.w]);
-                    }
-                    bending_eval<kDamp>(static_cast<int>(ref & 3u), x0, x1, x2, x3, p0, p1, p2, p3, em, inv_dt, f, h);
+                    float th = kNoAngle;
+                    if (kDamp && em.w > 0.0f)
+                        th = hinge_angle(xyz(s_prev[hi.x]), xyz(s_prev[hi.y]), xyz(s_prev[hi.z]), xyz(s_prev[hi.w]));
+                    bending_eval<kDamp>(static_cast<int>(ref & 3u), x0, x1, x2, x3, th, em.x, em.z * em.y, em.w * em.y,
+                                        inv_dt, f, h);
                 }
             }
             f.x = lane_sum(f.x);

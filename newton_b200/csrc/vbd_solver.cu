@@ -88,7 +88,8 @@ struct SolverImpl {
     long long steps = 0;
     int last_step_kernels = -1;  // kernel launches of the last vbd_step (graph kernel nodes; -1: not a graph)
     int staged_iteration = 0;    // iteration of the staged API (vbd_forward resets, vbd_begin_iteration sets)
-    // scratch (allocated once at create)
+    // scratch (allocated once at create, as one block)
+    unsigned char* arena = nullptr;
     float4* pos = nullptr;    // Gauss-Seidel iterate (state_in.particle_q in the reference)
     float4* prev = nullptr;   // particle_q_prev == pos_prev_collision_detection (step start)
     float4* y = nullptr;      // inertia target, .w = mass
@@ -96,6 +97,8 @@ struct SolverImpl {
     int* ccount = nullptr;    // [V] contacts per vertex (internal order)
     int* cslot = nullptr;     // [V*K] record ids
     float4* ctab = nullptr;   // [V*K][4] the step's contacts per vertex, packed and in record order
+    float4* tri_c = nullptr;     // [n_tri_rec] F^T F of each record's triangle at the step's start (damping)
+    float* edge_th = nullptr;    // [n_edge_rec] angle of each record's hinge at the step's start (damping)
     unsigned* status = nullptr;  // [kStatusSlots]
     float* resid_max = nullptr;  // [1] scratch for vbd_residual
     cudaStream_t capture_stream = nullptr;
@@ -152,6 +155,41 @@ namespace vbd {
 // ---------------------------------------------------------------------------------------------
 // kernels
 // ---------------------------------------------------------------------------------------------
+// Damping compares with the step's start: each triangle record's F^T F and each hinge record's angle
+// there are the same for all sweeps of the step, so they are computed once per step -- by the forward
+// pass, or by prepare_kernel when the step has contacts to pack -- instead of gathering and evaluating
+// the step-start positions again in every sweep (two or three gathers and 30 to 60 instructions per
+// record become one coalesced load).  With branch-free hinges (bending_eval), 10 iterations take
+// 334 -> 304 us at 65,536 vertices (membrane damping), 273 -> 230 at 22,500 (both), 6.05 -> 5.56 ms at
+// 1.89 M.
+struct StepTables {
+    const int4* vadj;
+    const int4* tri_idx;
+    const float4* tri_D;
+    const int4* edge_idx;
+    const float* edge_kd;  // NULL: no bending damping
+    float4* tri_c;         // NULL: no damping, or a caller without room for the tables
+    float* edge_th;
+};
+
+constexpr int kTableLanes = 4;  // lanes per vertex while the tables are written
+
+// vertex i's records; pos(j): step-start position of internal vertex j
+template <typename Pos>
+__device__ __forceinline__ void write_tables(const StepTables& t, int i, int lane, Pos pos) {
+    const int4 adj = t.vadj[i];
+    for (int r = adj.x + lane; r < adj.y; r += kTableLanes) {
+        const int4 ti = t.tri_idx[r];
+        const float3 c = membrane_metric(pos(ti.x), pos(ti.y), pos(ti.z), t.tri_D[r]);
+        t.tri_c[r] = make_float4(c.x, c.y, c.z, 0.f);
+    }
+    if (!t.edge_kd) return;
+    for (int r = adj.z + lane; r < adj.w; r += kTableLanes) {
+        const int4 ei = t.edge_idx[r];
+        t.edge_th[r] = hinge_angle(pos(ei.x & 0x3fffffff), pos(ei.y), pos(ei.z), pos(ei.w));
+    }
+}
+
 struct ForwardArgs {
     const int* perm;
     const int* inv_perm;
@@ -174,12 +212,19 @@ struct ForwardArgs {
     int* cslot;
     int K;
     unsigned* status;
+    StepTables tables;  // written here when tri_c is set: kTableLanes threads per vertex, lane 0 its state
 };
 
 __global__ void forward_kernel(ForwardArgs a) {
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (tid < a.V) {
-        const int i = tid;
+    const int lanes = a.tables.tri_c ? kTableLanes : 1;
+    if (a.tables.tri_c && tid / kTableLanes < a.V)
+        write_tables(a.tables, tid / kTableLanes, tid % kTableLanes, [&](int j) {
+            const int o = a.perm[j];
+            return f3(a.q_in[3 * o], a.q_in[3 * o + 1], a.q_in[3 * o + 2]);
+        });
+    if (tid / lanes < a.V && tid % lanes == 0) {
+        const int i = tid / lanes;
         const int o = a.perm[i];
         const float4 pi = a.pinfo[i];
         const int flags = __float_as_int(pi.w);
@@ -217,13 +262,14 @@ __global__ void forward_kernel(ForwardArgs a) {
     }
 }
 
-// Per-step packing of the contact table: the scatter above leaves each vertex's record ids in
-// arbitrary (atomic) order; this pass sorts them (the reference adds a particle's contacts in
-// record order) and gathers what the contact law reads into 4 float4 per contact:
+// Per-step preparation after the forward pass of a step with contacts, kTableLanes lanes per vertex:
+// the damping tables, and by lane 0 the contact table.  The scatter above leaves each vertex's record
+// ids in arbitrary (atomic) order; they are sorted (the reference adds a particle's contacts in record
+// order) and what the contact law reads is gathered into 4 float4 per contact:
 //   (body_pos, ke) (body_vel, kd) (normal, mu) (margin, 0, 0, 0)
 // so that every color sweep of the step reads one contiguous entry per contact instead of the
 // id -> record -> shape chain.
-struct PackArgs {
+struct PrepareArgs {
     const int* ccount;
     const int* cslot;
     int K;
@@ -233,12 +279,12 @@ struct PackArgs {
     const float* c_normal;
     const DevShape* shapes;
     float4* ctab;
+    const float4* prev;
+    StepTables tables;
     int V;
 };
 
-__global__ void pack_contacts_kernel(PackArgs a) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.V) return;
+__device__ __forceinline__ void pack_contacts(const PrepareArgs& a, int i) {
     const int n = min(a.ccount[i], a.K);
     if (n <= 0) return;
     // K <= 8: odd-even transposition sort of 8 slots (unused slots hold INT_MAX and sort last);
@@ -269,6 +315,14 @@ __global__ void pack_contacts_kernel(PackArgs a) {
     }
 }
 
+__global__ void prepare_kernel(PrepareArgs a) {
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = tid / kTableLanes, lane = tid % kTableLanes;
+    if (i >= a.V) return;
+    if (a.tables.tri_c) write_tables(a.tables, i, lane, [&](int j) { return xyz(a.prev[j]); });
+    if (lane == 0) pack_contacts(a, i);
+}
+
 // What a residual check needs besides the state (baked into the step graph).
 struct GateParams {
     float tol;
@@ -293,7 +347,10 @@ struct SweepArgs {
     const float4* tri_D;
     const float4* tri_mat;
     const int4* edge_idx;
-    const float4* edge_mat;
+    const float2* edge_mat;
+    const float* edge_kd;
+    const float4* tri_c;     // damping: the step-start metrics and angles (write_tables)
+    const float* edge_th;
     // contacts
     const int* ccount;
     const int* cslot;
@@ -303,7 +360,7 @@ struct SweepArgs {
     const float* c_body_vel;
     const float* c_normal;
     const DevShape* shapes;
-    // packed contact table (pack_contacts_kernel); NULL: read the records through cslot instead
+    // packed contact table (prepare_kernel); NULL: read the records through cslot instead
     const float4* ctab;
     // self-contact force / Hessian of the vertex (NULL without self-contact)
     const float4* sc_f;
@@ -335,117 +392,133 @@ struct SweepArgs {
     int patch_base;
 };
 
-// The staged positions of a block: [patch size] iterate positions, then (damping) [patch size]
-// step-start positions.
+// The staged positions of a block: [patch size] iterate positions.
 extern __shared__ float4 s_stage[];
 
-template <bool kDamp>
-__device__ __forceinline__ void accumulate_elements(const SweepArgs& a, int i, int lane, int L, int4 adj, float3& f,
-                                                    Sym3& h) {
-    // the vertex's records are dealt round-robin over one merged list (triangles, then hinges),
-    // so every lane gets the same number of records to within one
+// How a sweep damps (template parameter): not at all; the membrane; membrane and hinges -- both with
+// the step-start metrics and angles of prepare_kernel; or both from the step-start positions, for a
+// caller without room for those tables (vbd_step_static).  All give the same bits.
+enum Damping { kDampNone = 0, kDampTri = 1, kDampAll = 2, kDampDirect = 3 };
+
+// One triangle / hinge record: what a lane loads (in one go, so that the loads of two records can be
+// in flight together), and its evaluation.  kStaged: positions from the block's shared-memory patch
+// through the record's local indices, else from global memory.
+struct TriRecord {
+    float3 x0, x1, x2, c;
+    float4 D, m;
+    int slot;
+};
+
+template <int kDamp, bool kStaged>
+__device__ __forceinline__ TriRecord load_tri(const SweepArgs& a, int r, const float4* s_pos) {
+    TriRecord t;
+    int i0, i1, i2;
+    if (kStaged) {
+        const uint2 l = __ldg(&a.tri_loc[r]);
+        i0 = l.x & 0xffff;
+        i1 = l.x >> 16;
+        i2 = l.y & 0xffff;
+        t.slot = l.y >> 16;
+    } else {
+        const int4 n = __ldg(&a.tri_idx[r]);
+        i0 = n.x;
+        i1 = n.y;
+        i2 = n.z;
+        t.slot = n.w;
+    }
+    t.D = __ldg(&a.tri_D[r]);
+    t.m = __ldg(&a.tri_mat[r]);
+    t.c = f3(0.f, 0.f, 0.f);
+    if (kDamp == kDampTri || kDamp == kDampAll) t.c = xyz(__ldg(&a.tri_c[r]));
+    t.x0 = xyz(kStaged ? s_pos[i0] : a.pos[i0]);
+    t.x1 = xyz(kStaged ? s_pos[i1] : a.pos[i1]);
+    t.x2 = xyz(kStaged ? s_pos[i2] : a.pos[i2]);
+    if (kDamp == kDampDirect && t.m.w > 0.0f)
+        t.c = membrane_metric(xyz(__ldg(&a.prev[i0])), xyz(__ldg(&a.prev[i1])), xyz(__ldg(&a.prev[i2])), t.D);
+    return t;
+}
+
+struct HingeRecord {
+    float3 x0, x1, x2, x3;
+    float2 m;
+    float kd, th;
+    int order;
+};
+
+template <int kDamp, bool kStaged>
+__device__ __forceinline__ HingeRecord load_hinge(const SweepArgs& a, int r, const float4* s_pos) {
+    HingeRecord t;
+    int i0, i1, i2, i3;
+    if (kStaged) {
+        const uint2 l = __ldg(&a.edge_loc[r]);
+        i0 = l.x & 0x3fff;
+        t.order = (l.x >> 14) & 3;
+        i1 = l.x >> 16;
+        i2 = l.y & 0xffff;
+        i3 = l.y >> 16;
+    } else {
+        const int4 n = __ldg(&a.edge_idx[r]);
+        t.order = static_cast<int>(static_cast<unsigned>(n.x) >> 30);
+        i0 = n.x & 0x3fffffff;
+        i1 = n.y;
+        i2 = n.z;
+        i3 = n.w;
+    }
+    t.m = __ldg(&a.edge_mat[r]);
+    t.kd = 0.f;
+    t.th = kNoAngle;
+    if (kDamp == kDampAll) {
+        t.kd = __ldg(&a.edge_kd[r]);
+        t.th = __ldg(&a.edge_th[r]);
+    }
+    t.x0 = xyz(kStaged ? s_pos[i0] : a.pos[i0]);
+    t.x1 = xyz(kStaged ? s_pos[i1] : a.pos[i1]);
+    t.x2 = xyz(kStaged ? s_pos[i2] : a.pos[i2]);
+    t.x3 = xyz(kStaged ? s_pos[i3] : a.pos[i3]);
+    if (kDamp == kDampDirect && a.edge_kd) {
+        t.kd = __ldg(&a.edge_kd[r]);
+        if (t.kd > 0.0f)
+            t.th = hinge_angle(xyz(__ldg(&a.prev[i0])), xyz(__ldg(&a.prev[i1])), xyz(__ldg(&a.prev[i2])),
+                               xyz(__ldg(&a.prev[i3])));
+    }
+    return t;
+}
+
+template <int kDamp>
+__device__ __forceinline__ void add_tri(const SweepArgs& a, const TriRecord& t, float3& f, Sym3& h) {
+    membrane_eval<kDamp != kDampNone>(t.slot, t.x0, t.x1, t.x2, t.c, t.D, t.m, a.inv_dt, f, h);
+}
+template <int kDamp>
+__device__ __forceinline__ void add_hinge(const SweepArgs& a, const HingeRecord& t, float3& f, Sym3& h) {
+    bending_eval<(kDamp >= kDampAll)>(t.order, t.x0, t.x1, t.x2, t.x3, t.th, t.m.x, t.m.y, t.kd, a.inv_dt, f, h);
+}
+
+// A lane's share of its vertex's records, dealt round-robin over one merged list (triangles, then
+// hinges), so every lane gets the same number of records to within one.
+// kTwo: two records in flight per lane: records r and r + L are loaded and evaluated as two
+// independent chains (zero-started partial sums, added in record order), so the latency of one
+// record's loads and math overlaps the other's.  Used where the launch leaves registers for it (few
+// lanes per vertex, uncapped build).  A lane with an odd count evaluates its last record twice and
+// keeps one result.
+template <int kDamp, bool kStaged, bool kTwo>
+__device__ __forceinline__ void accumulate_elements(const SweepArgs& a, int lane, int L, int4 adj, const float4* s_pos,
+                                                    float3& f, Sym3& h) {
     const int nt = adj.y - adj.x;
     const int lane_e = (lane - nt % L + L) % L;  // first hinge slot of this lane
-    for (int r = adj.x + lane; r < adj.y; r += L) {
-        const int4 ti = __ldg(&a.tri_idx[r]);
-        const float4 D = __ldg(&a.tri_D[r]);
-        const float4 mt = __ldg(&a.tri_mat[r]);
-        const float3 x0 = xyz(a.pos[ti.x]), x1 = xyz(a.pos[ti.y]), x2 = xyz(a.pos[ti.z]);
-        float3 p0 = x0, p1 = x1, p2 = x2;
-        if (kDamp && mt.w > 0.0f) {
-            p0 = xyz(__ldg(&a.prev[ti.x]));
-            p1 = xyz(__ldg(&a.prev[ti.y]));
-            p2 = xyz(__ldg(&a.prev[ti.z]));
-        }
-        membrane_eval<kDamp>(ti.w, x0, x1, x2, p0, p1, p2, D, mt, a.inv_dt, f, h);
+    if (!kTwo) {
+        for (int r = adj.x + lane; r < adj.y; r += L) add_tri<kDamp>(a, load_tri<kDamp, kStaged>(a, r, s_pos), f, h);
+        for (int r = adj.z + lane_e; r < adj.w; r += L)
+            add_hinge<kDamp>(a, load_hinge<kDamp, kStaged>(a, r, s_pos), f, h);
+        return;
     }
-    for (int r = adj.z + lane_e; r < adj.w; r += L) {
-        const int4 ei = __ldg(&a.edge_idx[r]);
-        const float4 em = __ldg(&a.edge_mat[r]);
-        const int order = static_cast<int>(static_cast<unsigned>(ei.x) >> 30);
-        const int o0 = ei.x & 0x3fffffff;
-        const float3 x0 = xyz(a.pos[o0]), x1 = xyz(a.pos[ei.y]), x2 = xyz(a.pos[ei.z]), x3 = xyz(a.pos[ei.w]);
-        float3 p0 = x0, p1 = x1, p2 = x2, p3 = x3;
-        if (kDamp && em.w > 0.0f) {
-            p0 = xyz(__ldg(&a.prev[o0]));
-            p1 = xyz(__ldg(&a.prev[ei.y]));
-            p2 = xyz(__ldg(&a.prev[ei.z]));
-            p3 = xyz(__ldg(&a.prev[ei.w]));
-        }
-        bending_eval<kDamp>(order, x0, x1, x2, x3, p0, p1, p2, p3, em, a.inv_dt, f, h);
-    }
-}
-
-// The staged walk: the same records and the same math, with every position read from the block's
-// shared-memory patch (s_pos, and s_prev for damping) through the record's local indices.
-template <bool kDamp>
-__device__ __forceinline__ void accumulate_elements_staged(const SweepArgs& a, int lane, int L, int4 adj,
-                                                           const float4* s_pos, const float4* s_prev, float3& f,
-                                                           Sym3& h) {
-    const int nt = adj.y - adj.x;
-    const int lane_e = (lane - nt % L + L) % L;
-    for (int r = adj.x + lane; r < adj.y; r += L) {
-        const uint2 tl = __ldg(&a.tri_loc[r]);
-        const float4 D = __ldg(&a.tri_D[r]);
-        const float4 mt = __ldg(&a.tri_mat[r]);
-        const int l0 = tl.x & 0xffff, l1 = tl.x >> 16, l2 = tl.y & 0xffff, slot = tl.y >> 16;
-        const float3 x0 = xyz(s_pos[l0]), x1 = xyz(s_pos[l1]), x2 = xyz(s_pos[l2]);
-        float3 p0 = x0, p1 = x1, p2 = x2;
-        if (kDamp && mt.w > 0.0f) {
-            p0 = xyz(s_prev[l0]);
-            p1 = xyz(s_prev[l1]);
-            p2 = xyz(s_prev[l2]);
-        }
-        membrane_eval<kDamp>(slot, x0, x1, x2, p0, p1, p2, D, mt, a.inv_dt, f, h);
-    }
-    for (int r = adj.z + lane_e; r < adj.w; r += L) {
-        const uint2 el = __ldg(&a.edge_loc[r]);
-        const float4 em = __ldg(&a.edge_mat[r]);
-        const int o0 = el.x & 0x3fff, order = (el.x >> 14) & 3, o1 = el.x >> 16, v0 = el.y & 0xffff, v1 = el.y >> 16;
-        const float3 x0 = xyz(s_pos[o0]), x1 = xyz(s_pos[o1]), x2 = xyz(s_pos[v0]), x3 = xyz(s_pos[v1]);
-        float3 p0 = x0, p1 = x1, p2 = x2, p3 = x3;
-        if (kDamp && em.w > 0.0f) {
-            p0 = xyz(s_prev[o0]);
-            p1 = xyz(s_prev[o1]);
-            p2 = xyz(s_prev[v0]);
-            p3 = xyz(s_prev[v1]);
-        }
-        bending_eval<kDamp>(order, x0, x1, x2, x3, p0, p1, p2, p3, em, a.inv_dt, f, h);
-    }
-}
-
-// The staged walk with two records in flight per lane: accumulate_elements_x2's order and math,
-// positions from the patch (used where the unstaged sweep uses the two-record walk, so that both
-// give the same bits).
-template <bool kDamp>
-__device__ __forceinline__ void accumulate_elements_staged_x2(const SweepArgs& a, int lane, int L, int4 adj,
-                                                              const float4* s_pos, const float4* s_prev, float3& f,
-                                                              Sym3& h) {
-    const int nt = adj.y - adj.x;
-    const int lane_e = (lane - nt % L + L) % L;
     for (int r = adj.x + lane; r < adj.y; r += 2 * L) {
         const bool two = r + L < adj.y;
-        const int rb = two ? r + L : r;
-        const uint2 ta = __ldg(&a.tri_loc[r]), tb = __ldg(&a.tri_loc[rb]);
-        const float4 Da = __ldg(&a.tri_D[r]), Db = __ldg(&a.tri_D[rb]);
-        const float4 ma = __ldg(&a.tri_mat[r]), mb = __ldg(&a.tri_mat[rb]);
-        const int a0 = ta.x & 0xffff, a1 = ta.x >> 16, a2 = ta.y & 0xffff, sa = ta.y >> 16;
-        const int b0 = tb.x & 0xffff, b1 = tb.x >> 16, b2 = tb.y & 0xffff, sb = tb.y >> 16;
-        const float3 xa0 = xyz(s_pos[a0]), xa1 = xyz(s_pos[a1]), xa2 = xyz(s_pos[a2]);
-        const float3 xb0 = xyz(s_pos[b0]), xb1 = xyz(s_pos[b1]), xb2 = xyz(s_pos[b2]);
-        float3 pa0 = xa0, pa1 = xa1, pa2 = xa2, pb0 = xb0, pb1 = xb1, pb2 = xb2;
-        if (kDamp && (ma.w > 0.0f || mb.w > 0.0f)) {
-            pa0 = xyz(s_prev[a0]);
-            pa1 = xyz(s_prev[a1]);
-            pa2 = xyz(s_prev[a2]);
-            pb0 = xyz(s_prev[b0]);
-            pb1 = xyz(s_prev[b1]);
-            pb2 = xyz(s_prev[b2]);
-        }
+        const TriRecord ta = load_tri<kDamp, kStaged>(a, r, s_pos);
+        const TriRecord tb = load_tri<kDamp, kStaged>(a, two ? r + L : r, s_pos);
         float3 fa = f3(0.f, 0.f, 0.f), fb = fa;
         Sym3 ha = zero_sym(), hb = zero_sym();
-        membrane_eval<kDamp>(sa, xa0, xa1, xa2, pa0, pa1, pa2, Da, ma, a.inv_dt, fa, ha);
-        membrane_eval<kDamp>(sb, xb0, xb1, xb2, pb0, pb1, pb2, Db, mb, a.inv_dt, fb, hb);
+        add_tri<kDamp>(a, ta, fa, ha);
+        add_tri<kDamp>(a, tb, fb, hb);
         f = f + fa;
         add(h, ha);
         if (two) {
@@ -455,100 +528,12 @@ __device__ __forceinline__ void accumulate_elements_staged_x2(const SweepArgs& a
     }
     for (int r = adj.z + lane_e; r < adj.w; r += 2 * L) {
         const bool two = r + L < adj.w;
-        const int rb = two ? r + L : r;
-        const uint2 ea = __ldg(&a.edge_loc[r]), eb = __ldg(&a.edge_loc[rb]);
-        const float4 ma = __ldg(&a.edge_mat[r]), mb = __ldg(&a.edge_mat[rb]);
-        const int oa = (ea.x >> 14) & 3, ob = (eb.x >> 14) & 3;
-        const int a0 = ea.x & 0x3fff, a1 = ea.x >> 16, a2 = ea.y & 0xffff, a3 = ea.y >> 16;
-        const int b0 = eb.x & 0x3fff, b1 = eb.x >> 16, b2 = eb.y & 0xffff, b3 = eb.y >> 16;
-        const float3 xa0 = xyz(s_pos[a0]), xa1 = xyz(s_pos[a1]), xa2 = xyz(s_pos[a2]), xa3 = xyz(s_pos[a3]);
-        const float3 xb0 = xyz(s_pos[b0]), xb1 = xyz(s_pos[b1]), xb2 = xyz(s_pos[b2]), xb3 = xyz(s_pos[b3]);
-        float3 pa0 = xa0, pa1 = xa1, pa2 = xa2, pa3 = xa3, pb0 = xb0, pb1 = xb1, pb2 = xb2, pb3 = xb3;
-        if (kDamp && (ma.w > 0.0f || mb.w > 0.0f)) {
-            pa0 = xyz(s_prev[a0]);
-            pa1 = xyz(s_prev[a1]);
-            pa2 = xyz(s_prev[a2]);
-            pa3 = xyz(s_prev[a3]);
-            pb0 = xyz(s_prev[b0]);
-            pb1 = xyz(s_prev[b1]);
-            pb2 = xyz(s_prev[b2]);
-            pb3 = xyz(s_prev[b3]);
-        }
+        const HingeRecord ta = load_hinge<kDamp, kStaged>(a, r, s_pos);
+        const HingeRecord tb = load_hinge<kDamp, kStaged>(a, two ? r + L : r, s_pos);
         float3 fa = f3(0.f, 0.f, 0.f), fb = fa;
         Sym3 ha = zero_sym(), hb = zero_sym();
-        bending_eval<kDamp, true>(oa, xa0, xa1, xa2, xa3, pa0, pa1, pa2, pa3, ma, a.inv_dt, fa, ha);
-        bending_eval<kDamp, true>(ob, xb0, xb1, xb2, xb3, pb0, pb1, pb2, pb3, mb, a.inv_dt, fb, hb);
-        f = f + fa;
-        add(h, ha);
-        if (two) {
-            f = f + fb;
-            add(h, hb);
-        }
-    }
-}
-
-// The same walk with two records in flight per lane: records r and r + L are loaded and evaluated
-// as two independent chains (zero-started partial sums, added in record order), so the latency of
-// one record's loads and math overlaps the other's.  Used where the launch leaves registers for
-// it (few lanes per vertex, uncapped build).  A lane with an odd count evaluates its last record
-// twice and keeps one result.
-template <bool kDamp>
-__device__ __forceinline__ void accumulate_elements_x2(const SweepArgs& a, int lane, int L, int4 adj, float3& f,
-                                                       Sym3& h) {
-    const int nt = adj.y - adj.x;
-    const int lane_e = (lane - nt % L + L) % L;
-    for (int r = adj.x + lane; r < adj.y; r += 2 * L) {
-        const bool two = r + L < adj.y;
-        const int rb = two ? r + L : r;
-        const int4 ta = __ldg(&a.tri_idx[r]), tb = __ldg(&a.tri_idx[rb]);
-        const float4 Da = __ldg(&a.tri_D[r]), Db = __ldg(&a.tri_D[rb]);
-        const float4 ma = __ldg(&a.tri_mat[r]), mb = __ldg(&a.tri_mat[rb]);
-        const float3 xa0 = xyz(a.pos[ta.x]), xa1 = xyz(a.pos[ta.y]), xa2 = xyz(a.pos[ta.z]);
-        const float3 xb0 = xyz(a.pos[tb.x]), xb1 = xyz(a.pos[tb.y]), xb2 = xyz(a.pos[tb.z]);
-        float3 pa0 = xa0, pa1 = xa1, pa2 = xa2, pb0 = xb0, pb1 = xb1, pb2 = xb2;
-        if (kDamp && (ma.w > 0.0f || mb.w > 0.0f)) {
-            pa0 = xyz(__ldg(&a.prev[ta.x]));
-            pa1 = xyz(__ldg(&a.prev[ta.y]));
-            pa2 = xyz(__ldg(&a.prev[ta.z]));
-            pb0 = xyz(__ldg(&a.prev[tb.x]));
-            pb1 = xyz(__ldg(&a.prev[tb.y]));
-            pb2 = xyz(__ldg(&a.prev[tb.z]));
-        }
-        float3 fa = f3(0.f, 0.f, 0.f), fb = fa;
-        Sym3 ha = zero_sym(), hb = zero_sym();
-        membrane_eval<kDamp>(ta.w, xa0, xa1, xa2, pa0, pa1, pa2, Da, ma, a.inv_dt, fa, ha);
-        membrane_eval<kDamp>(tb.w, xb0, xb1, xb2, pb0, pb1, pb2, Db, mb, a.inv_dt, fb, hb);
-        f = f + fa;
-        add(h, ha);
-        if (two) {
-            f = f + fb;
-            add(h, hb);
-        }
-    }
-    for (int r = adj.z + lane_e; r < adj.w; r += 2 * L) {
-        const bool two = r + L < adj.w;
-        const int rb = two ? r + L : r;
-        const int4 ea = __ldg(&a.edge_idx[r]), eb = __ldg(&a.edge_idx[rb]);
-        const float4 ma = __ldg(&a.edge_mat[r]), mb = __ldg(&a.edge_mat[rb]);
-        const int oa = static_cast<int>(static_cast<unsigned>(ea.x) >> 30), ob = static_cast<int>(static_cast<unsigned>(eb.x) >> 30);
-        const int a0 = ea.x & 0x3fffffff, b0 = eb.x & 0x3fffffff;
-        const float3 xa0 = xyz(a.pos[a0]), xa1 = xyz(a.pos[ea.y]), xa2 = xyz(a.pos[ea.z]), xa3 = xyz(a.pos[ea.w]);
-        const float3 xb0 = xyz(a.pos[b0]), xb1 = xyz(a.pos[eb.y]), xb2 = xyz(a.pos[eb.z]), xb3 = xyz(a.pos[eb.w]);
-        float3 pa0 = xa0, pa1 = xa1, pa2 = xa2, pa3 = xa3, pb0 = xb0, pb1 = xb1, pb2 = xb2, pb3 = xb3;
-        if (kDamp && (ma.w > 0.0f || mb.w > 0.0f)) {
-            pa0 = xyz(__ldg(&a.prev[a0]));
-            pa1 = xyz(__ldg(&a.prev[ea.y]));
-            pa2 = xyz(__ldg(&a.prev[ea.z]));
-            pa3 = xyz(__ldg(&a.prev[ea.w]));
-            pb0 = xyz(__ldg(&a.prev[b0]));
-            pb1 = xyz(__ldg(&a.prev[eb.y]));
-            pb2 = xyz(__ldg(&a.prev[eb.z]));
-            pb3 = xyz(__ldg(&a.prev[eb.w]));
-        }
-        float3 fa = f3(0.f, 0.f, 0.f), fb = fa;
-        Sym3 ha = zero_sym(), hb = zero_sym();
-        bending_eval<kDamp, true>(oa, xa0, xa1, xa2, xa3, pa0, pa1, pa2, pa3, ma, a.inv_dt, fa, ha);
-        bending_eval<kDamp, true>(ob, xb0, xb1, xb2, xb3, pb0, pb1, pb2, pb3, mb, a.inv_dt, fb, hb);
+        add_hinge<kDamp>(a, ta, fa, ha);
+        add_hinge<kDamp>(a, tb, fb, hb);
         f = f + fa;
         add(h, ha);
         if (two) {
@@ -584,13 +569,13 @@ __device__ __forceinline__ void prefetch_l2(const void* p) {
     asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
-// L2 prefetch of the 128-byte lines holding records [b, e) of a 16-byte-per-record array, the
-// lines dealt round-robin over the vertex's L lanes
-__device__ __forceinline__ void prefetch_rows_l2(const void* base, int b, int e, int lane, int L) {
+// L2 prefetch of the 128-byte lines holding records [b, e), the lines dealt round-robin over the
+// vertex's L lanes
+template <typename T>
+__device__ __forceinline__ void prefetch_rows_l2(const T* base, int b, int e, int lane, int L) {
     if (e <= b) return;
-    const char* p = static_cast<const char*>(base);
-    const uintptr_t first = reinterpret_cast<uintptr_t>(p + 16 * static_cast<size_t>(b)) & ~uintptr_t(127);
-    const uintptr_t last = reinterpret_cast<uintptr_t>(p + 16 * static_cast<size_t>(e) - 1) & ~uintptr_t(127);
+    const uintptr_t first = reinterpret_cast<uintptr_t>(base + b) & ~uintptr_t(127);
+    const uintptr_t last = (reinterpret_cast<uintptr_t>(base + e) - 1) & ~uintptr_t(127);
     for (uintptr_t line = first + 128 * static_cast<uintptr_t>(lane); line <= last; line += 128 * static_cast<uintptr_t>(L))
         prefetch_l2(reinterpret_cast<const void*>(line));
 }
@@ -771,7 +756,7 @@ __device__ __forceinline__ void reduce_residual_lanes(const SweepArgs& a, float 
 // Hessian are summed across the L lanes with xor shuffles and lane 0 adds the contacts and solves.
 // kCap: the same kernel limited to 64 registers per thread (4 blocks of 256 per SM), used when the
 // uncapped kernel would need more than one wave of blocks (large colors, many lanes per vertex)
-template <int L, bool kDamp, bool kResidual, bool kCap, bool kGate, bool kStaged = false>
+template <int L, int kDamp, bool kResidual, bool kCap, bool kGate, bool kStaged = false>
 __device__ __forceinline__ void sweep_body(const SweepArgs& a) {
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = a.v_begin + tid / L;
@@ -806,21 +791,13 @@ __device__ __forceinline__ void sweep_body(const SweepArgs& a) {
     // an earlier kernel of the stream and is the same for every thread of the grid)
     if (a.gate_stop && *reinterpret_cast<const volatile unsigned*>(a.gate_stop) != 0u) return;
     const float4* s_pos = s_stage;
-    const float4* s_prev = s_stage;
     if (kStaged) {
         // the block's one-ring: one coalesced pass over the patch ids, one gather per position
         // (the previous kernel's writes are visible after griddepcontrol.wait), then every record
         // of the block reads its positions from shared memory
         const int p = a.patch_base + static_cast<int>(blockIdx.x);
         const int b0 = __ldg(&a.patch_off[p]), n = __ldg(&a.patch_off[p + 1]) - b0;
-        float4* sp = s_stage;
-        float4* sq = s_stage + n;
-        for (int j = threadIdx.x; j < n; j += blockDim.x) {
-            const int g = __ldg(&a.patch_ids[b0 + j]);
-            sp[j] = a.pos[g];
-            if (kDamp) sq[j] = __ldg(&a.prev[g]);
-        }
-        s_prev = sq;
+        for (int j = threadIdx.x; j < n; j += blockDim.x) s_stage[j] = a.pos[__ldg(&a.patch_ids[b0 + j])];
         __syncthreads();
     }
     if (valid && solve && lane == 0) {
@@ -841,10 +818,7 @@ __device__ __forceinline__ void sweep_body(const SweepArgs& a) {
         }
     }
     if (valid && solve) {
-        if (kStaged && L <= 2 && !kCap) accumulate_elements_staged_x2<kDamp>(a, lane, L, adj, s_pos, s_prev, f, h);
-        else if (kStaged) accumulate_elements_staged<kDamp>(a, lane, L, adj, s_pos, s_prev, f, h);
-        else if (L <= 2 && !kCap) accumulate_elements_x2<kDamp>(a, lane, L, adj, f, h);
-        else accumulate_elements<kDamp>(a, i, lane, L, adj, f, h);
+        accumulate_elements<kDamp, kStaged, (L <= 2 && !kCap)>(a, lane, L, adj, s_pos, f, h);
     }
     if (L > 1) {
         f.x = warp_sum(f.x, L);
@@ -911,7 +885,7 @@ __device__ __forceinline__ void sweep_body(const SweepArgs& a) {
     solve_and_commit(a, i, pv, h, f);
 }
 
-template <int L, bool kDamp, bool kResidual, bool kCap, bool kGate = false, bool kStaged = false>
+template <int L, int kDamp, bool kResidual, bool kCap, bool kGate = false, bool kStaged = false>
 __global__ void __launch_bounds__(256, kCap ? 4 : 1) sweep_kernel(SweepArgs a) {
     sweep_body<L, kDamp, kResidual, kCap, kGate, kStaged>(a);
 }
@@ -920,14 +894,14 @@ __global__ void __launch_bounds__(256, kCap ? 4 : 1) sweep_kernel(SweepArgs a) {
 // plain sweep: at 74 (what the compiler picks for the extra reduction) the allocation rounds up
 // to 80 registers per thread, two color grids no longer fit on an SM together, and each launch
 // loses its overlap with the previous one.
-template <int L, bool kDamp, bool kStaged = false>
+template <int L, int kDamp, bool kStaged = false>
 __global__ void __maxnreg__(72) sweep_gate_kernel(SweepArgs a) {
     sweep_body<L, kDamp, false, false, true, kStaged>(a);
 }
 
 // The staged sweep at 4 or more lanes, held to the same 72 registers (unbounded, the damping
 // build takes 79).
-template <int L, bool kDamp>
+template <int L, int kDamp>
 __global__ void __maxnreg__(72) sweep_staged_kernel(SweepArgs a) {
     sweep_body<L, kDamp, false, false, false, true>(a);
 }
@@ -941,7 +915,7 @@ __global__ void __maxnreg__(72) sweep_staged_kernel(SweepArgs a) {
 // (solve_elasticity, particle_vbd_kernels.py:2568-2706): inertia, triangles in CSR order, hinges
 // in CSR order, then the accumulated contact force and Hessian.  The order never depends on
 // thread scheduling, so results are deterministic.
-template <int TB, bool kDamp, bool kResidual>
+template <int TB, int kDamp, bool kResidual>
 __global__ void __launch_bounds__(TB) tile_kernel(SweepArgs a) {
     constexpr int VT = TB / 16;
     constexpr int MAXR = 2 * TB;
@@ -985,36 +959,8 @@ __global__ void __launch_bounds__(TB) tile_kernel(SweepArgs a) {
             float3 f = f3(0.f, 0.f, 0.f);
             Sym3 h = zero_sym();
             const int k = base + r;
-            if (k < nt) {
-                const int rec = tb + k;
-                const int4 ti = __ldg(&a.tri_idx[rec]);
-                const float4 D = __ldg(&a.tri_D[rec]);
-                const float4 mt = __ldg(&a.tri_mat[rec]);
-                const float3 x0 = xyz(a.pos[ti.x]), x1 = xyz(a.pos[ti.y]), x2 = xyz(a.pos[ti.z]);
-                float3 p0 = x0, p1 = x1, p2 = x2;
-                if (kDamp && mt.w > 0.0f) {
-                    p0 = xyz(__ldg(&a.prev[ti.x]));
-                    p1 = xyz(__ldg(&a.prev[ti.y]));
-                    p2 = xyz(__ldg(&a.prev[ti.z]));
-                }
-                membrane_eval<kDamp>(ti.w, x0, x1, x2, p0, p1, p2, D, mt, a.inv_dt, f, h);
-            } else {
-                const int rec = eb + (k - nt);
-                const int4 ei = __ldg(&a.edge_idx[rec]);
-                const float4 em = __ldg(&a.edge_mat[rec]);
-                const int order = static_cast<int>(static_cast<unsigned>(ei.x) >> 30);
-                const int o0 = ei.x & 0x3fffffff;
-                const float3 x0 = xyz(a.pos[o0]), x1 = xyz(a.pos[ei.y]), x2 = xyz(a.pos[ei.z]),
-                             x3 = xyz(a.pos[ei.w]);
-                float3 p0 = x0, p1 = x1, p2 = x2, p3 = x3;
-                if (kDamp && em.w > 0.0f) {
-                    p0 = xyz(__ldg(&a.prev[o0]));
-                    p1 = xyz(__ldg(&a.prev[ei.y]));
-                    p2 = xyz(__ldg(&a.prev[ei.z]));
-                    p3 = xyz(__ldg(&a.prev[ei.w]));
-                }
-                bending_eval<kDamp>(order, x0, x1, x2, x3, p0, p1, p2, p3, em, a.inv_dt, f, h);
-            }
+            if (k < nt) add_tri<kDamp>(a, load_tri<kDamp, false>(a, tb + k, nullptr), f, h);
+            else add_hinge<kDamp>(a, load_hinge<kDamp, false>(a, eb + (k - nt), nullptr), f, h);
             s_c[0 * STRIDE + r] = f.x;
             s_c[1 * STRIDE + r] = f.y;
             s_c[2 * STRIDE + r] = f.z;
@@ -1236,6 +1182,9 @@ static SweepArgs make_sweep_args(const SolverImpl& s, const VbdContacts* c, floa
     a.tri_mat = m.tri_mat;
     a.edge_idx = m.edge_idx;
     a.edge_mat = m.edge_mat;
+    a.edge_kd = m.edge_kd;
+    a.tri_c = s.tri_c;
+    a.edge_th = s.edge_th;
     a.K = s.K;
     if (c && m.S > 0) {
         a.ccount = s.ccount;
@@ -1336,7 +1285,7 @@ static void launch_gate(void (*kernel)(Args...), cudaStream_t st, bool pdl, Args
 
 // the staged instantiations: the same choice between the uncapped (or 72-register gate) kernel
 // and the 64-register one, with the patch's shared memory counted in the occupancy
-template <int L, bool kDamp, bool kGate>
+template <int L, int kDamp, bool kGate>
 static void launch_staged_LDG(const SweepArgs& a, int grid, int block, cudaStream_t st, size_t smem) {
     if constexpr (kGate && L >= 4) {
         if (grid > resident_blocks(reinterpret_cast<const void*>(&sweep_gate_kernel<L, kDamp, true>), block, smem))
@@ -1358,27 +1307,27 @@ static void launch_staged_LDG(const SweepArgs& a, int grid, int block, cudaStrea
     }
 }
 
-template <int L>
-static void prime_staged_occupancy_L(int block, size_t smem) {
+template <int L, int kDamp>
+static void prime_staged_occupancy_LD(int block, size_t smem) {
     if constexpr (L >= 4) {
-        resident_blocks(reinterpret_cast<const void*>(&sweep_staged_kernel<L, true>), block, smem);
-        resident_blocks(reinterpret_cast<const void*>(&sweep_staged_kernel<L, false>), block, smem);
+        resident_blocks(reinterpret_cast<const void*>(&sweep_staged_kernel<L, kDamp>), block, smem);
+        resident_blocks(reinterpret_cast<const void*>(&sweep_gate_kernel<L, kDamp, true>), block, smem);
     } else {
-        resident_blocks(reinterpret_cast<const void*>(&sweep_kernel<L, true, false, false, false, true>), block, smem);
-        resident_blocks(reinterpret_cast<const void*>(&sweep_kernel<L, false, false, false, false, true>), block, smem);
-    }
-    if constexpr (L >= 4) {
-        resident_blocks(reinterpret_cast<const void*>(&sweep_gate_kernel<L, true, true>), block, smem);
-        resident_blocks(reinterpret_cast<const void*>(&sweep_gate_kernel<L, false, true>), block, smem);
-    } else {
-        resident_blocks(reinterpret_cast<const void*>(&sweep_kernel<L, true, false, false, true, true>), block, smem);
-        resident_blocks(reinterpret_cast<const void*>(&sweep_kernel<L, false, false, false, true, true>), block, smem);
+        resident_blocks(reinterpret_cast<const void*>(&sweep_kernel<L, kDamp, false, false, false, true>), block, smem);
+        resident_blocks(reinterpret_cast<const void*>(&sweep_kernel<L, kDamp, false, false, true, true>), block, smem);
     }
 }
 
-template <int L, bool kDamp, bool kResidual, bool kGate = false>
+template <int L>
+static void prime_staged_occupancy_L(int block, size_t smem) {
+    prime_staged_occupancy_LD<L, kDampNone>(block, smem);
+    prime_staged_occupancy_LD<L, kDampTri>(block, smem);
+    prime_staged_occupancy_LD<L, kDampAll>(block, smem);
+}
+
+template <int L, int kDamp, bool kResidual, bool kGate = false>
 static void launch_sweep_LDR(const SweepArgs& a, int grid, int block, cudaStream_t st, size_t smem = 0) {
-    if constexpr (!kResidual) {
+    if constexpr (!kResidual && kDamp != kDampDirect) {
         if (a.patch_off) {
             launch_staged_LDG<L, kDamp, kGate>(a, grid, block, st, smem);
             return;
@@ -1399,18 +1348,20 @@ static void launch_sweep_LDR(const SweepArgs& a, int grid, int block, cudaStream
 }
 
 // occupancy queries happen here, outside any stream capture (solver creation, vbd_set_launch)
+template <int L, int kDamp>
+static void prime_occupancy_LD(int block) {
+    resident_blocks(reinterpret_cast<const void*>(&sweep_kernel<L, kDamp, true, false>), block);
+    resident_blocks(reinterpret_cast<const void*>(&sweep_kernel<L, kDamp, false, false>), block);
+    resident_blocks(reinterpret_cast<const void*>(&sweep_kernel<L, kDamp, false, false, true>), block);
+    if constexpr (L >= 4) resident_blocks(reinterpret_cast<const void*>(&sweep_gate_kernel<L, kDamp>), block);
+}
+
 template <int L>
 static void prime_occupancy_L(int block) {
-    resident_blocks(reinterpret_cast<const void*>(&sweep_kernel<L, true, true, false>), block);
-    resident_blocks(reinterpret_cast<const void*>(&sweep_kernel<L, false, true, false>), block);
-    resident_blocks(reinterpret_cast<const void*>(&sweep_kernel<L, true, false, false>), block);
-    resident_blocks(reinterpret_cast<const void*>(&sweep_kernel<L, false, false, false>), block);
-    resident_blocks(reinterpret_cast<const void*>(&sweep_kernel<L, true, false, false, true>), block);
-    resident_blocks(reinterpret_cast<const void*>(&sweep_kernel<L, false, false, false, true>), block);
-    if constexpr (L >= 4) {
-        resident_blocks(reinterpret_cast<const void*>(&sweep_gate_kernel<L, true>), block);
-        resident_blocks(reinterpret_cast<const void*>(&sweep_gate_kernel<L, false>), block);
-    }
+    prime_occupancy_LD<L, kDampNone>(block);
+    prime_occupancy_LD<L, kDampTri>(block);
+    prime_occupancy_LD<L, kDampAll>(block);
+    if constexpr (L == 4) resident_blocks(reinterpret_cast<const void*>(&sweep_kernel<L, kDampDirect, false, false>), block);
 }
 
 static void prime_occupancy(int lanes, int block) {
@@ -1424,42 +1375,56 @@ static void prime_occupancy(int lanes, int block) {
     }
 }
 
+template <int L, int kDamp>
+static void launch_sweep_LD(const SweepArgs& a, bool residual, int grid, int block, cudaStream_t st, bool gate,
+                            size_t smem) {
+    if (residual) launch_sweep_LDR<L, kDamp, true>(a, grid, block, st);
+    else if (gate) launch_sweep_LDR<L, kDamp, false, true>(a, grid, block, st, smem);
+    else launch_sweep_LDR<L, kDamp, false>(a, grid, block, st, smem);
+}
+
 template <int L>
-static void launch_sweep_L(const SweepArgs& a, bool damp, bool residual, int block, cudaStream_t st, bool gate,
+static void launch_sweep_L(const SweepArgs& a, int damp, bool residual, int block, cudaStream_t st, bool gate,
                            size_t smem) {
     const long long threads = static_cast<long long>(a.v_end - a.v_begin) * L;
     const int grid = static_cast<int>((threads + block - 1) / block);
     if (grid <= 0) return;
-    if (gate && !residual) {
-        if (damp) launch_sweep_LDR<L, true, false, true>(a, grid, block, st, smem);
-        else launch_sweep_LDR<L, false, false, true>(a, grid, block, st, smem);
-        return;
+    if constexpr (L == 4) {
+        if (damp == kDampDirect) {  // vbd_step_static: plain sweeps of the default shape
+            launch_sweep_LDR<L, kDampDirect, false>(a, grid, block, st);
+            return;
+        }
     }
-    if (residual) {
-        if (damp) launch_sweep_LDR<L, true, true>(a, grid, block, st);
-        else launch_sweep_LDR<L, false, true>(a, grid, block, st);
-    } else {
-        if (damp) launch_sweep_LDR<L, true, false>(a, grid, block, st, smem);
-        else launch_sweep_LDR<L, false, false>(a, grid, block, st, smem);
-    }
+    if (damp == kDampNone) launch_sweep_LD<L, kDampNone>(a, residual, grid, block, st, gate, smem);
+    else if (damp == kDampTri) launch_sweep_LD<L, kDampTri>(a, residual, grid, block, st, gate, smem);
+    else launch_sweep_LD<L, kDampAll>(a, residual, grid, block, st, gate, smem);
 }
 
-template <int TB>
-static void launch_tile_TB(const SweepArgs& a, bool damp, bool residual, cudaStream_t st) {
+template <int TB, int kDamp>
+static void launch_tile_TBD(const SweepArgs& a, bool residual, cudaStream_t st) {
     constexpr int VT = TB / 16;
     const int grid = (a.v_end - a.v_begin + VT - 1) / VT;
     if (grid <= 0) return;
-    if (residual) {
-        if (damp) tile_kernel<TB, true, true><<<grid, TB, 0, st>>>(a);
-        else tile_kernel<TB, false, true><<<grid, TB, 0, st>>>(a);
-    } else {
-        if (damp) tile_kernel<TB, true, false><<<grid, TB, 0, st>>>(a);
-        else tile_kernel<TB, false, false><<<grid, TB, 0, st>>>(a);
-    }
+    if (residual) tile_kernel<TB, kDamp, true><<<grid, TB, 0, st>>>(a);
+    else tile_kernel<TB, kDamp, false><<<grid, TB, 0, st>>>(a);
+}
+
+template <int TB>
+static void launch_tile_TB(const SweepArgs& a, int damp, bool residual, cudaStream_t st) {
+    if (damp == kDampNone) launch_tile_TBD<TB, kDampNone>(a, residual, st);
+    else if (damp == kDampTri) launch_tile_TBD<TB, kDampTri>(a, residual, st);
+    else launch_tile_TBD<TB, kDampAll>(a, residual, st);
+}
+
+static int damping_of(const SolverImpl& s) {
+    const VbdModelImpl& m = *s.m;
+    if (!m.any_tri_damping && !m.any_edge_damping) return kDampNone;
+    if (!s.tri_c) return kDampDirect;
+    return m.any_edge_damping ? kDampAll : kDampTri;
 }
 
 // gate: a Gauss-Seidel color that also accumulates its residual into a.resid_* (lanes > 0 only)
-static void launch_sweep(const SweepArgs& a, int lanes, bool damp, bool residual, int block, cudaStream_t st,
+static void launch_sweep(const SweepArgs& a, int lanes, int damp, bool residual, int block, cudaStream_t st,
                          bool gate = false, size_t smem = 0) {
     if (lanes == 0) {
         if (block <= 64) launch_tile_TB<64>(a, damp, residual, st);
@@ -1477,7 +1442,7 @@ static void launch_sweep(const SweepArgs& a, int lanes, bool damp, bool residual
 }
 
 static int enqueue_forward(SolverImpl& s, const float* q_in, const float* qd_in, const float* f_ext,
-                           const VbdContacts* c, float dt, cudaStream_t st) {
+                           const VbdContacts* c, float dt, cudaStream_t st, bool tables = true) {
     const VbdModelImpl& m = *s.m;
     s.last_dt = dt;
     ForwardArgs a;
@@ -1510,10 +1475,17 @@ static int enqueue_forward(SolverImpl& s, const float* q_in, const float* qd_in,
         // autotuner runs -- leaves it set)
         VBD_CUDA_TRY(cudaMemsetAsync(s.ccount, 0, sizeof(int) * static_cast<size_t>(m.V), st));
     }
+    const bool pack = a.c_count && s.ctab && m.V > 0;
+    StepTables t;
+    std::memset(&t, 0, sizeof(t));
+    if (tables && s.tri_c) t = {m.vadj, m.tri_idx, m.tri_D, m.edge_idx, m.edge_kd, s.tri_c, s.edge_th};
+    if (!pack) a.tables = t;
     const int block = 256;
-    if (n > 0) forward_kernel<<<(n + block - 1) / block, block, 0, st>>>(a);
-    if (a.c_count && s.ctab && m.V > 0) {
-        PackArgs p;
+    const long long threads = static_cast<long long>(m.V) * kTableLanes;
+    auto grid = [block](long long k) { return static_cast<unsigned>((k + block - 1) / block); };
+    if (n > 0) forward_kernel<<<grid(a.tables.tri_c ? std::max<long long>(n, threads) : n), block, 0, st>>>(a);
+    if (pack) {
+        PrepareArgs p;
         p.ccount = s.ccount;
         p.cslot = s.cslot;
         p.K = s.K;
@@ -1523,8 +1495,10 @@ static int enqueue_forward(SolverImpl& s, const float* q_in, const float* qd_in,
         p.c_normal = c->soft_contact_normal;
         p.shapes = m.shapes;
         p.ctab = s.ctab;
+        p.prev = s.prev;
+        p.tables = t;
         p.V = m.V;
-        pack_contacts_kernel<<<(m.V + block - 1) / block, block, 0, st>>>(p);
+        prepare_kernel<<<grid(threads), block, 0, st>>>(p);
     }
     return VBD_OK;
 }
@@ -1545,18 +1519,18 @@ static void enqueue_color(SolverImpl& s, int color, const VbdContacts* c, float 
     a.v_end = m.color_start[color + 1];
     if (a.v_end <= a.v_begin) return;
     size_t smem = 0;
-    const bool damp = m.any_tri_damping || m.any_edge_damping;
+    const int damp = damping_of(s);
     if (s.stage_on && s.stage_ready && !s.sc.on && s.lanes == s.stage_lanes && s.block == s.stage_block) {
         a.patch_off = s.patch_off;
         a.patch_ids = s.patch_ids;
         a.tri_loc = s.tri_loc;
         a.edge_loc = s.edge_loc;
         a.patch_base = s.stage_color_base[color];
-        smem = static_cast<size_t>(s.stage_max_patch) * sizeof(float4) * (damp ? 2 : 1);
+        smem = static_cast<size_t>(s.stage_max_patch) * sizeof(float4);
     }
     if (s.sc.on) {
         self_contact_accumulate(m, s.sc, s.pos, s.prev, color, dt, s.friction_epsilon, st);
-        launch_sweep(a, s.lanes, m.any_tri_damping || m.any_edge_damping, false, s.block, st);
+        launch_sweep(a, s.lanes, damping_of(s), false, s.block, st);
         self_contact_truncate(m, s.sc, s.pos, s.disp, color, st);
         return;
     }
@@ -1649,7 +1623,7 @@ static void enqueue_gate_residual(SolverImpl& s, const VbdContacts* c, float dt,
     a.resid_out = nullptr;
     a.gate_max = s.gate_mean ? nullptr : s.gate->maxv;
     a.gate_sum = s.gate_mean ? s.gate->sum : nullptr;
-    launch_sweep(a, s.lanes, m.any_tri_damping || m.any_edge_damping, true, s.block, st);
+    launch_sweep(a, s.lanes, damping_of(s), true, s.block, st);
 }
 
 // The gated iterations of one step, recorded into the graph that `st` is capturing:
@@ -1721,7 +1695,8 @@ static int enqueue_gated_iterations(SolverImpl& s, const VbdContacts* c, float d
 
 static int enqueue_step(SolverImpl& s, float* q_in, const float* qd_in, const float* f_ext, float* q_out,
                         float* qd_out, const VbdContacts* c, float dt, int iterations, cudaStream_t st) {
-    enqueue_forward(s, q_in, qd_in, f_ext, c, dt, st);
+    const bool resident = s.resident_on && s.resident.ready && iterations > 0 && !(s.gate_tol > 0.f) && !s.ws_params;
+    enqueue_forward(s, q_in, qd_in, f_ext, c, dt, st, !resident);
     if (s.ws_params) {
         // learned warm start: features -> MLP -> iterate from y + prediction
         const bool gated = s.gate_tol > 0.f;
@@ -1747,7 +1722,7 @@ static int enqueue_step(SolverImpl& s, float* q_in, const float* qd_in, const fl
         enqueue_finalize(s, q_in, q_out, qd_out, dt, st, s.ws_corr);  // and the correction kept
         return VBD_OK;
     }
-    if (s.resident_on && s.resident.ready && iterations > 0 && !(s.gate_tol > 0.f)) {
+    if (resident) {
         const VbdModelImpl& m = *s.m;
         ResidentLaunch L;
         std::memset(&L, 0, sizeof(L));
@@ -1818,9 +1793,8 @@ static void free_solver(SolverImpl& s) {
     s.ws_corr = nullptr;
     for (auto& g : s.graphs) cudaGraphExecDestroy(g.exec);
     s.graphs.clear();
-    void* ptrs[] = {s.pos, s.prev, s.y, s.disp, s.ccount, s.cslot, s.ctab, s.status, s.resid_max};
-    for (void* p : ptrs)
-        if (p) cudaFree(p);
+    if (s.arena) cudaFree(s.arena);
+    s.arena = nullptr;
     if (s.capture_stream) cudaStreamDestroy(s.capture_stream);
     if (s.body_stream) cudaStreamDestroy(s.body_stream);
     if (s.gate) cudaFree(s.gate);
@@ -1829,6 +1803,8 @@ static void free_solver(SolverImpl& s) {
     s.pos = s.prev = s.y = s.disp = nullptr;
     s.ccount = s.cslot = nullptr;
     s.ctab = nullptr;
+    s.tri_c = nullptr;
+    s.edge_th = nullptr;
     s.status = nullptr;
     s.resid_max = nullptr;
     s.capture_stream = nullptr;
@@ -1892,23 +1868,41 @@ extern "C" int vbd_solver_create(const VbdModel* model, const VbdSolverOptions* 
         delete h;
         return fail(VBD_ERR_INVALID_ARGUMENT, "vbd_solver_create: contacts_per_vertex must be in [1, 8]");
     }
-    auto alloc = [&](void** p, size_t bytes) -> int {
-        if (bytes == 0) bytes = 16;
-        VBD_CUDA_TRY(cudaMalloc(p, bytes));
-        VBD_CUDA_TRY(cudaMemset(*p, 0, bytes));
-        return VBD_OK;
-    };
+    // one allocation for all of the solver's scratch, every array 256-byte aligned
     const size_t V = static_cast<size_t>(m.V);
+    const bool damped = m.any_tri_damping || m.any_edge_damping;
+    size_t bytes = 0;
+    auto place = [&](size_t n) {
+        const size_t at = bytes;
+        bytes += (std::max<size_t>(n, 16) + 255) & ~static_cast<size_t>(255);
+        return at;
+    };
+    const size_t o_pos = place(V * sizeof(float4)), o_prev = place(V * sizeof(float4)), o_y = place(V * sizeof(float4)),
+                 o_disp = place(V * sizeof(float4)), o_ccount = place(V * sizeof(int)),
+                 o_cslot = place(V * s.K * sizeof(int)), o_status = place(kStatusSlots * sizeof(unsigned)),
+                 o_resid = place(sizeof(float));
+    const size_t o_ctab = m.S > 0 ? place(V * s.K * 4 * sizeof(float4)) : 0;
+    const size_t o_tri_c = damped ? place(static_cast<size_t>(m.n_tri_rec) * sizeof(float4)) : 0;
+    const size_t o_edge_th = m.any_edge_damping ? place(static_cast<size_t>(m.n_edge_rec) * sizeof(float)) : 0;
     int rc = VBD_OK;
-    if (!rc) rc = alloc(reinterpret_cast<void**>(&s.pos), V * sizeof(float4));
-    if (!rc) rc = alloc(reinterpret_cast<void**>(&s.prev), V * sizeof(float4));
-    if (!rc) rc = alloc(reinterpret_cast<void**>(&s.y), V * sizeof(float4));
-    if (!rc) rc = alloc(reinterpret_cast<void**>(&s.disp), V * sizeof(float4));
-    if (!rc) rc = alloc(reinterpret_cast<void**>(&s.ccount), V * sizeof(int));
-    if (!rc) rc = alloc(reinterpret_cast<void**>(&s.cslot), V * s.K * sizeof(int));
-    if (!rc && m.S > 0) rc = alloc(reinterpret_cast<void**>(&s.ctab), V * s.K * 4 * sizeof(float4));
-    if (!rc) rc = alloc(reinterpret_cast<void**>(&s.status), kStatusSlots * sizeof(unsigned));
-    if (!rc) rc = alloc(reinterpret_cast<void**>(&s.resid_max), sizeof(float));
+    {
+        cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&s.arena), bytes);
+        if (e == cudaSuccess) e = cudaMemset(s.arena, 0, bytes);
+        if (e != cudaSuccess) rc = cuda_fail(e, "vbd_solver_create: scratch");
+    }
+    if (!rc) {
+        s.pos = reinterpret_cast<float4*>(s.arena + o_pos);
+        s.prev = reinterpret_cast<float4*>(s.arena + o_prev);
+        s.y = reinterpret_cast<float4*>(s.arena + o_y);
+        s.disp = reinterpret_cast<float4*>(s.arena + o_disp);
+        s.ccount = reinterpret_cast<int*>(s.arena + o_ccount);
+        s.cslot = reinterpret_cast<int*>(s.arena + o_cslot);
+        s.status = reinterpret_cast<unsigned*>(s.arena + o_status);
+        s.resid_max = reinterpret_cast<float*>(s.arena + o_resid);
+        if (m.S > 0) s.ctab = reinterpret_cast<float4*>(s.arena + o_ctab);
+        if (damped) s.tri_c = reinterpret_cast<float4*>(s.arena + o_tri_c);
+        if (m.any_edge_damping) s.edge_th = reinterpret_cast<float*>(s.arena + o_edge_th);
+    }
     if (!rc) {
         cudaError_t e = cudaStreamCreateWithFlags(&s.capture_stream, cudaStreamNonBlocking);
         if (e != cudaSuccess) rc = cuda_fail(e, "cudaStreamCreateWithFlags");
@@ -2276,7 +2270,7 @@ extern "C" int vbd_residual(VbdSolver* solver, const VbdContacts* contacts, floa
     a.v_end = m.swept;
     a.resid_out = per_vertex_out;
     a.resid_max = mx;
-    launch_sweep(a, s.lanes, m.any_tri_damping || m.any_edge_damping, true, s.block, st);
+    launch_sweep(a, s.lanes, damping_of(s), true, s.block, st);
     VBD_CUDA_TRY(cudaGetLastError());
     return VBD_OK;
 }
@@ -2387,7 +2381,7 @@ extern "C" int vbd_solver_info(const VbdSolver* solver, int32_t* color_count, in
 }
 
 // ---- staged sweep ---------------------------------------------------------------------------
-constexpr int kMaxPatch = 1536;  // patch entries: local indices fit 14 bits; 2 x 16 B x 1536 = 48 KB
+constexpr int kMaxPatch = 1536;  // patch entries: local indices fit 14 bits; 16 B x 1536 = 24 KB
 
 static void free_staged(SolverImpl& s) {
     cudaFree(s.patch_off);
@@ -2486,8 +2480,7 @@ static int build_staged(SolverImpl& s) {
     s.stage_block = s.block;
     s.stage_ready = true;
     // occupancy of the staged kernels with their shared memory, queried outside any capture
-    const bool damp = m.any_tri_damping || m.any_edge_damping;
-    const size_t smem = static_cast<size_t>(maxp) * sizeof(float4) * (damp ? 2 : 1);
+    const size_t smem = static_cast<size_t>(maxp) * sizeof(float4);
     switch (s.lanes) {
         case 1: prime_staged_occupancy_L<1>(s.block, smem); break;
         case 2: prime_staged_occupancy_L<2>(s.block, smem); break;
