@@ -125,7 +125,9 @@ typedef struct VbdModelDesc {
 typedef struct VbdSolverOptions {
     int32_t iterations;           /* default VBD iterations per step (reference default 10) */
     float friction_epsilon;       /* reference default 1e-2 */
-    int32_t lanes_per_vertex;     /* 1,2,4,8,16 = that many lanes cooperate on one vertex; 0 = default (4);
+    int32_t lanes_per_vertex;     /* 1,2,4,8,16 = that many lanes cooperate on one vertex; 0 = default: 16
+                                     or 8 for models without worlds whose largest color has at most 4,096 or
+                                     10,240 vertices, else 4 (vbd_solver_info reports it);
                                      -1 = record-parallel sweep (one thread per element record) */
     int32_t block_size;           /* threads per block of the sweep, 0 = default 128 (64/128/256 when
                                      lanes_per_vertex is 0) */
@@ -254,8 +256,8 @@ int vbd_batch_step(VbdSolver* const* solvers, int32_t count, float* const* q_in,
  * the library sized for at most 16384 particles (about 5.3 MiB, held on every GPU that loads the
  * library until the process exits); larger models are rejected with VBD_ERR_INVALID_ARGUMENT.
  * Allocates nothing and takes no solver: same arrays, aliasing and bit-identical results as
- * vbd_step of a solver with the default options (lanes_per_vertex 4, block_size 128, 4 contacts
- * per vertex, no self-contact, no warm start).  Call it with the model's device current (another
+ * vbd_step of a solver with lanes_per_vertex 4, block_size 128, 4 contacts per vertex, no
+ * self-contact and no warm start.  Call it with the model's device current (another
  * current device is rejected).  The first call on a device looks up the array's device address;
  * make that first call before any stream capture.  Every call shares the one array (it clears
  * the parts that must start at zero), so calls that overlap on the GPU -- concurrent streams or

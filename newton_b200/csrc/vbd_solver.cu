@@ -81,7 +81,7 @@ struct SolverImpl {
     const VbdModelImpl* m = nullptr;
     int iterations = 10;
     float friction_epsilon = 1e-2f;
-    int lanes = 4;  // 0: record-parallel tiles; 1..16: lanes cooperating on one vertex
+    int lanes = 4;  // 0: record-parallel tiles; 1..16: lanes cooperating on one vertex (default_lanes)
     int block = 128;
     int K = 4;
     bool use_graph = true;
@@ -1823,6 +1823,20 @@ static const char* launch_shape_error(int lanes, int block) {
     return nullptr;
 }
 
+// Lanes per vertex when the caller leaves the choice to the library.  A small color is a latency chain
+// over a vertex's records, and more lanes shorten it while the GPU has room: 10 iterations take, in
+// us with 4 / 8 / 16 lanes, 208 / 172 / 150 at 1,024 vertices, 240 / 193 / 178 at 9,216, 237 / 203 / 196
+// at 16,384 (4,096 per color), 232 / 197 / 207 at 22,500, 269 / 256 / 240 at 32,761 and, where 4
+// lanes fill it, 304 / 301 / 402 at 65,536, 465 / 597 / 824 at 129,600.
+// A model made of worlds keeps 4: the lane count decides the summation order, and a world's result
+// must not depend on how many others share its model (shards reproduce the whole bit for bit).
+static int default_lanes(const VbdModelImpl& m) {
+    if (m.n_worlds > 0) return 4;
+    int largest = 0;
+    for (int c = 0; c < m.C; ++c) largest = std::max(largest, m.color_start[c + 1] - m.color_start[c]);
+    return largest <= 4096 ? 16 : (largest <= 10240 ? 8 : 4);
+}
+
 static bool same_contacts(const VbdContacts& a, const VbdContacts& b) { return std::memcmp(&a, &b, sizeof(a)) == 0; }
 
 static int check_state_args(const char* fn, const float* a, const float* b) {
@@ -1842,6 +1856,7 @@ extern "C" int vbd_solver_create(const VbdModel* model, const VbdSolverOptions* 
     VbdSolver* h = new VbdSolver();
     SolverImpl& s = h->s;
     s.m = &m;
+    s.lanes = default_lanes(m);
     if (options) {
         if (options->iterations < 0) {
             delete h;
