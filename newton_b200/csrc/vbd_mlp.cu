@@ -502,7 +502,7 @@ static int tc_forward(const float* params, const float* X, int32_t n, float* Y, 
     a.off_b2 = kOffB2;
     a.off_w3 = kOffW3;
     a.off_b3 = kOffB3;
-    tc::mlp_infer_tc_kernel<tc::kInF32><<<tc_grid(n), tc::kThreads, tc::kSmemBytes, st>>>(a);
+    tc::mlp_infer_tc_kernel<tc::kInF32><<<tc_grid(n), tc::threads_of(tc::kInF32), tc::kSmemBytes, st>>>(a);
     VBD_CUDA_TRY(cudaGetLastError());
     return VBD_OK;
 }
@@ -549,7 +549,7 @@ int mlp_step_start(const VbdModelImpl& m, const float* params, const float4* pre
     a.off_b2 = kOffB2;
     a.off_w3 = kOffW3;
     a.off_b3 = kOffB3;
-    tc::mlp_infer_tc_kernel<tc::kInStep><<<tc_grid(m.V), tc::kThreads, tc::kSmemBytes, st>>>(a);
+    tc::mlp_infer_tc_kernel<tc::kInStep><<<tc_grid(m.V), tc::threads_of(tc::kInStep), tc::kSmemBytes, st>>>(a);
     VBD_CUDA_TRY(cudaGetLastError());
     return VBD_OK;
 }

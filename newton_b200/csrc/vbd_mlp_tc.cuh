@@ -2,10 +2,12 @@
 // generation tensor cores: tcgen05.mma with FP16 operands in shared memory and FP32 accumulators
 // in tensor memory (TMEM); bias + SiLU in f16x2 arithmetic.  Included by vbd_mlp.cu only.
 //
-// Work split.  One persistent CTA of 512 threads per SM runs four independent tile pipelines
-// ("groups" of 4 warps) over one shared copy of the weights.  A group owns one 128-row tile of
-// samples at a time; its warp q reads TMEM lanes [32 q, 32 q + 32), the rows of those samples, and
-// thread 32 q + l owns row 32 q + l.  Per tile, in the group's 32 KB operand buffer and its 128 TMEM
+// Work split.  One persistent CTA per SM runs four independent tile pipelines ("groups") over one
+// shared copy of the weights.  A group owns one 128-row tile of samples at a time; its warp q reads
+// TMEM lanes [32 (q % 4), + 32), the rows of those samples.  From feature rows in HBM a group has 8
+// warps, two per row quarter, each with half of the columns (1024 threads per SM: every step of a tile
+// is a short latency chain, so twice the warps with half the columns each cover more of it); in
+// the step mode 4 warps, one thread per row, which computes the row's 64 features in registers.  Per tile, in the group's 32 KB operand buffer and its 128 TMEM
 // columns:
 //   1. the group stages the tile's features as FP16 (128 x 64, the first 16 KB of the buffer), read
 //      from FP32 rows or, in the step mode, computed from the solver's arrays;
@@ -44,8 +46,6 @@ namespace tc {
 
 constexpr int kRows = 128;                   // samples per tile (MMA M, TMEM lanes)
 constexpr int kGroups = 4;                   // tile pipelines per CTA
-constexpr int kGroupThreads = 128;           // 4 warps, one per TMEM lane quarter
-constexpr int kThreads = kGroups * kGroupThreads;
 constexpr uint32_t kTmemCols = 512;          // 128 per group: D of layer 1, then of layer 2, then 3
 constexpr unsigned kTcSpinLimit = 1u << 26;  // polls of one mbarrier wait before giving up
 
@@ -130,19 +130,23 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
 
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-// barrier of one group's 128 threads (named barrier 1 + group; 0 is the CTA-wide __syncthreads)
-__device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
+// barrier of one group's threads (named barrier 1 + group; 0 is the CTA-wide __syncthreads)
+template <int kCount>
+__device__ __forceinline__ void group_sync(int id) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kCount) : "memory");
+}
 
-// the group's threads agree: true only if `v` is true in all 128
+// the group's threads agree: true only if `v` is true in all of them
+template <int kCount>
 __device__ __forceinline__ bool group_all(int id, bool v) {
     uint32_t r;
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.u32 p, %1, 0;\n\t"
-        "bar.red.and.pred q, %2, 128, p;\n\t"
+        "bar.red.and.pred q, %2, %3, p;\n\t"
         "selp.u32 %0, 1, 0, q;\n\t}\n"
         : "=r"(r)
-        : "r"(v ? 1u : 0u), "r"(id)
+        : "r"(v ? 1u : 0u), "r"(id), "n"(kCount)
         : "memory");
     return r != 0;
 }
@@ -170,6 +174,23 @@ __device__ __forceinline__ void tmem_ld64(uint32_t taddr, float (&v)[64]) {
     for (int j = 0; j < 64; ++j) v[j] = __uint_as_float(r[j]);
 }
 
+// 32 consecutive FP32 columns of this thread's TMEM lane (one load, one wait)
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
+    uint32_t r[32];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr)
+        : "memory");
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+}
+
 // two FP32 values rounded to nearest FP16, packed (lo in the low half)
 __device__ __forceinline__ uint32_t pack_f16(float lo, float hi) {
     __half2 v = __floats2half2_rn(lo, hi);
@@ -192,13 +213,14 @@ __device__ __forceinline__ uint32_t silu2_bias_f16(float z0, float z1, uint32_t 
     return *reinterpret_cast<uint32_t*>(&out);
 }
 
-// bias + SiLU of 64 accumulator columns [c0, c0 + 64) of row r, stored as FP16 into an R = 128 row
-// K-major operand (8 stores of 16 bytes); the bias is read 8 values at a time (a broadcast: every
+// bias + SiLU of N accumulator columns [c0, c0 + N) of row r, stored as FP16 into an R = 128 row
+// K-major operand (stores of 16 bytes); the bias is read 8 values at a time (a broadcast: every
 // thread of the warp reads the same address)
-__device__ __forceinline__ void store_hidden64(unsigned char* A, int r, int c0, const float (&acc)[64],
-                                               const uint32_t* bias2) {
+template <int N>
+__device__ __forceinline__ void store_hidden(unsigned char* A, int r, int c0, const float (&acc)[N],
+                                             const uint32_t* bias2) {
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
+    for (int q = 0; q < N / 8; ++q) {
         const uint4 b = *reinterpret_cast<const uint4*>(bias2 + (c0 + q * 8) / 2);  // 8 biases, FP16 pairs
         const float* x = acc + q * 8;
         uint4 w;
@@ -388,8 +410,26 @@ __device__ __forceinline__ void stage_step_row(const TcStep& s, int i, int n, co
     }
 }
 
+constexpr int split_of(int input) { return input == kInF32 ? 2 : 1; }            // warps per row quarter
+constexpr int threads_of(int input) { return kGroups * kRows * split_of(input); }  // of the CTA
+
+// columns [c_begin, c_end) of the accumulator: bias, SiLU, FP16, into the next layer's operand
+template <int kChunk>
+__device__ __forceinline__ void hidden_epilogue(uint32_t d, unsigned char* buf, int r, int c_begin, int c_end,
+                                                const uint32_t* bias2) {
+#pragma unroll 1
+    for (int c0 = c_begin; c0 < c_end; c0 += kChunk) {
+        float acc[kChunk];
+        if constexpr (kChunk == 64) tmem_ld64(d + c0, acc);
+        else tmem_ld32(d + c0, acc);
+        store_hidden<kChunk>(buf, r, c0, acc, bias2);
+    }
+}
+
 template <int kInput>
-__global__ void __launch_bounds__(kThreads, 1) mlp_infer_tc_kernel(TcArgs a) {
+__global__ void __launch_bounds__(threads_of(kInput), 1) mlp_infer_tc_kernel(TcArgs a) {
+    constexpr int kSplit = split_of(kInput), kThreads = threads_of(kInput), kGroupThreads = kRows * kSplit;
+    constexpr int kChunk = kSplit == 2 ? 32 : 64;  // accumulator columns in registers at a time
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     unsigned char* sW1 = smem + kOffW1;
@@ -403,7 +443,9 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_infer_tc_kernel(TcArgs a) {
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kOffBar);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kOffBar + 8 * kGroups);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int group = warp >> 2, quarter = warp & 3, gtid = tid & (kGroupThreads - 1);
+    const int group = tid / kGroupThreads, gtid = tid % kGroupThreads;
+    const int quarter = warp & 3, part = (gtid >> 5) >> 2;  // row quarter (TMEM lanes), column part
+    const int c_begin = part * (128 / kSplit), c_end = c_begin + 128 / kSplit;
     const int bar_id = 1 + group;
     unsigned char* buf = smem + kOffBuf + group * kSzBuf;
     const uint32_t bar = smem_u32(bars + group);
@@ -459,10 +501,11 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_infer_tc_kernel(TcArgs a) {
 
     for (int tile = blockIdx.x * kGroups + group; tile < ntiles; tile += gridDim.x * kGroups) {
         const int row0 = tile * kRows;
-        // ---- 1. features -> the buffer as FP16.  Warp q stages rows [32 q, 32 q + 32): in pass j
-        // a lane takes row 32 q + 8 (j / 4) + lane % 8 and float4 column 4 (j % 4) + lane / 8, so each
-        // load reads 8 rows x 64 contiguous bytes and each store fills whole core-matrix rows; the
-        // 16 loads are in flight together (the other groups' work covers their latency) ----
+        // ---- 1. features -> the buffer as FP16.  The warps of quarter q stage rows [32 q, 32 q + 32)
+        // in 16 passes (a part of them each): in pass j a lane takes row 32 q + 8 (j / 4) + lane % 8 and
+        // float4 column 4 (j % 4) + lane / 8, so each load reads 8 rows x 64 contiguous bytes and each
+        // store fills whole core-matrix rows; a warp's loads are in flight together (the other groups'
+        // work covers their latency) ----
         if (kInput == kInStep) {
             // this thread's row: its features from the solver's arrays (one-ring gathers; the other
             // groups' MMAs and epilogues cover their latency)
@@ -471,28 +514,31 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_infer_tc_kernel(TcArgs a) {
             else
                 stage_step_row<false>(a.step, row0 + r_own, a.n, normalize ? sMean : nullptr, sIstd, buf, r_own);
         } else {
-            float4 v[16];
+            constexpr int kPasses = 16 / kSplit;
+            float4 v[kPasses];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
+            for (int k = 0; k < kPasses; ++k) {
+                const int j = part * kPasses + k;
                 const int r = quarter * 32 + 8 * (j >> 2) + (lane & 7);
                 const int c4 = 4 * (j & 3) + (lane >> 3);
-                v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (row0 + r < a.n)
-                    v[j] = __ldg(reinterpret_cast<const float4*>(a.X + static_cast<size_t>(row0 + r) * 64) + c4);
+                    v[k] = __ldg(reinterpret_cast<const float4*>(a.X + static_cast<size_t>(row0 + r) * 64) + c4);
             }
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
+            for (int k = 0; k < kPasses; ++k) {
+                const int j = part * kPasses + k;
                 const int r = quarter * 32 + 8 * (j >> 2) + (lane & 7);
                 const int c4 = 4 * (j & 3) + (lane >> 3);
                 uint2 w;
-                w.x = pack_f16(v[j].x, v[j].y);
-                w.y = pack_f16(v[j].z, v[j].w);
+                w.x = pack_f16(v[k].x, v[k].y);
+                w.y = pack_f16(v[k].z, v[k].w);
                 *reinterpret_cast<uint2*>(buf + kmajor_offset(r, 4 * c4, kRows)) = w;
             }
         }
         fence_proxy_async();
         fence_before();
-        group_sync(bar_id);
+        group_sync<kGroupThreads>(bar_id);
         if (kInput == kInStep) {
             // the group's next tile: its rows' own data toward L2 while this tile runs (a prefetch
             // holds no register; measured 4-5% off the launch at 1.89 M rows)
@@ -516,19 +562,14 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_infer_tc_kernel(TcArgs a) {
                          s > 0 ? 1u : 0u);
             mma_commit(bar);
         }
-        ok = group_all(bar_id, bar_wait(bar, phase));  // one decision for the whole group
+        ok = group_all<kGroupThreads>(bar_id, bar_wait(bar, phase));  // one decision for the whole group
         if (!ok) break;
         phase ^= 1u;
         fence_after();
-#pragma unroll 1
-        for (int c0 = 0; c0 < 128; c0 += 64) {
-            float acc[64];
-            tmem_ld64(d + lane_base + c0, acc);
-            store_hidden64(buf, r_own, c0, acc, sB1);  // layer 1's MMAs have completed: X is free
-        }
+        hidden_epilogue<kChunk>(d + lane_base, buf, r_own, c_begin, c_end, sB1);  // layer 1's MMAs have completed: X is free
         fence_proxy_async();
         fence_before();
-        group_sync(bar_id);
+        group_sync<kGroupThreads>(bar_id);
         // ---- 3. layer 2 (D's columns reused: layer 1's epilogue has read them) ----
         if (issuer) {
             fence_after();
@@ -538,19 +579,14 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_infer_tc_kernel(TcArgs a) {
                          s > 0 ? 1u : 0u);
             mma_commit(bar);
         }
-        ok = group_all(bar_id, bar_wait(bar, phase));
+        ok = group_all<kGroupThreads>(bar_id, bar_wait(bar, phase));
         if (!ok) break;
         phase ^= 1u;
         fence_after();
-#pragma unroll 1
-        for (int c0 = 0; c0 < 128; c0 += 64) {
-            float acc[64];
-            tmem_ld64(d + lane_base + c0, acc);
-            store_hidden64(buf, r_own, c0, acc, sB2);  // layer 2's MMAs have completed: H1 is free
-        }
+        hidden_epilogue<kChunk>(d + lane_base, buf, r_own, c_begin, c_end, sB2);  // layer 2's MMAs have completed: H1 is free
         fence_proxy_async();
         fence_before();
-        group_sync(bar_id);
+        group_sync<kGroupThreads>(bar_id);
         // ---- 4. layer 3 ----
         if (issuer) {
             fence_after();
@@ -560,11 +596,11 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_infer_tc_kernel(TcArgs a) {
                          s > 0 ? 1u : 0u);
             mma_commit(bar);
         }
-        ok = group_all(bar_id, bar_wait(bar, phase));
+        ok = group_all<kGroupThreads>(bar_id, bar_wait(bar, phase));
         if (!ok) break;
         phase ^= 1u;
         fence_after();
-        {
+        if (part == 0) {
             float y[16];
             tmem_ld16(d + lane_base, y);
             const int r = row0 + r_own;
@@ -581,7 +617,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_infer_tc_kernel(TcArgs a) {
             }
         }
         fence_before();
-        group_sync(bar_id);  // the buffer and D are free for the group's next tile
+        group_sync<kGroupThreads>(bar_id);  // the buffer and D are free for the group's next tile
     }
     if (!ok) {
         // a wait gave up: record it, then wait (bounded) for the MMAs the group issued before the
