@@ -21,6 +21,14 @@
 
 namespace vbd {
 
+constexpr int kReachUnbounded = 255;
+
+// the byte bound of a displacement of length l (NaN: unbounded)
+__device__ __forceinline__ unsigned char reach_of(float l, float inv_unit) {
+    const float u = ceilf(l * inv_unit * 1.0001f);
+    return static_cast<unsigned char>(u <= 254.0f ? static_cast<int>(u) : kReachUnbounded);
+}
+
 struct SelfContactParams {
     float radius = 0.2f;
     float margin = 0.2f;
@@ -43,6 +51,10 @@ struct SelfContact {
     int V = 0, T = 0, E = 0;
     float cell = 0.f;       // grid cell edge
     float max_disp = 0.f;   // margin * relaxation * 0.5
+    // [V] |displacement from cd| of each vertex in units of reach_unit, rounded up (kReachUnbounded:
+    // beyond the range): an upper bound a byte wide, for the force pass's early rejection
+    unsigned char* reach = nullptr;
+    float reach_unit = 0.f;
     int tcap = 32;          // colliding vertices kept per triangle
     unsigned tri_mask = 0, edge_mask = 0;
     int tri_items_cap = 0, edge_items_cap = 0;
@@ -111,6 +123,8 @@ int self_contact_accumulate(const VbdModelImpl& m, SelfContact& sc, const float4
 // changed: those of `color` (-1: every vertex) and those that a plane shortens.
 int self_contact_truncate(const VbdModelImpl& m, SelfContact& sc, float4* pos, float4* disp, int color,
                           cudaStream_t st);
+// The byte bounds of all displacements (after something else than a sweep changed them).
+int self_contact_refresh_reach(const VbdModelImpl& m, SelfContact& sc, const float4* disp, cudaStream_t st);
 // Whether iteration `it` begins with a detection (particle_collision_detection_interval).
 bool self_contact_detect_now(const SelfContact& sc, int it);
 // Loads model-order positions [V,3] into cd (internal order) -- for detection from a given state.

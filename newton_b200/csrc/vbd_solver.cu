@@ -367,6 +367,8 @@ struct SweepArgs {
     const float4* sc_f;
     const float4* sc_h0;
     const float4* sc_h1;
+    unsigned char* sc_reach;  // bound of the vertex's displacement (SelfContact::reach)
+    float sc_reach_inv;
     // constants
     float dt, inv_dt, dt_sqr_recip, eps_u;
     unsigned* status;
@@ -640,6 +642,7 @@ __device__ __forceinline__ void solve_and_commit(const SweepArgs& a, int i, floa
         atomicAdd(&a.status[kSingular], 1u);
     }
     if (a.write_pos) a.pos[i] = make_float4(pv.x + d.x, pv.y + d.y, pv.z + d.z, 0.f);
+    if (a.sc_reach) a.sc_reach[i] = reach_of(length(xyz(d)), a.sc_reach_inv);
 }
 
 // Fixed-point scale of the residual sums (units of m|g|): r is rounded to 1/256 and clamped at
@@ -1049,6 +1052,7 @@ __global__ void __launch_bounds__(TB) tile_kernel(SweepArgs a) {
         atomicAdd(&a.status[kSingular], 1u);
     }
     if (a.write_pos) a.pos[i] = make_float4(pv.x + d.x, pv.y + d.y, pv.z + d.z, 0.f);
+    if (a.sc_reach) a.sc_reach[i] = reach_of(length(xyz(d)), a.sc_reach_inv);
 }
 
 // Commit of a color when the coloring is not conflict-free for every element stencil: the
@@ -1208,6 +1212,8 @@ static SweepArgs make_sweep_args(const SolverImpl& s, const VbdContacts* c, floa
         a.sc_f = s.sc.sc_f;
         a.sc_h0 = s.sc.sc_h0;
         a.sc_h1 = s.sc.sc_h1;
+        a.sc_reach = s.sc.reach;
+        a.sc_reach_inv = 1.0f / s.sc.reach_unit;
         a.write_pos = 0;
     }
     a.perm = m.perm;
@@ -2270,6 +2276,7 @@ extern "C" int vbd_warm_start(VbdSolver* solver, const float* delta, void* strea
     warm_start_kernel<<<(s.m->V + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(
         s.m->perm, s.m->pinfo, s.prev, s.disp, s.pos, delta, s.m->V);
     VBD_CUDA_TRY(cudaGetLastError());
+    if (s.sc.on) return self_contact_refresh_reach(*s.m, s.sc, s.disp, static_cast<cudaStream_t>(stream));
     return VBD_OK;
 }
 
