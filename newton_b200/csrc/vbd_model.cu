@@ -210,7 +210,7 @@ static int build_model(const VbdModelDesc* d, VbdModelImpl& m) {
     std::vector<float4> tri_D(n_tri_rec), tri_mat(n_tri_rec);
     std::vector<int4> edge_idx(n_edge_rec);
     std::vector<float4> edge_mat(n_edge_rec);
-    std::vector<float2> edge_rk(n_edge_rec);
+    std::vector<float2> edge_rk(n_edge_rec + 1);  // (one more: 16-byte copies may end past the last)
     std::vector<float> edge_kd(n_edge_rec);
     m.tri_elem_h.assign(n_tri_rec, 0);
     m.edge_elem_h.assign(n_edge_rec, 0);
