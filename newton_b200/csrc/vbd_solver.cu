@@ -226,8 +226,10 @@ __global__ void forward_kernel(ForwardArgs a) {
             return f3(a.q_in[3 * o], a.q_in[3 * o + 1], a.q_in[3 * o + 2]);
         });
     if (tid / lanes < a.V && tid % lanes == 0) {
-        const int i = tid / lanes;
-        const int o = a.perm[i];
+        // threads follow the model order where they can: consecutive particles alternate between few
+        // colors, so both sides of the reordering are read and written in runs
+        const int o = lanes == 1 ? tid : a.perm[tid / lanes];
+        const int i = lanes == 1 ? a.inv_perm[tid] : tid / lanes;
         const float4 pi = a.pinfo[i];
         const int flags = __float_as_int(pi.w);
         const float3 q = f3(a.q_in[3 * o], a.q_in[3 * o + 1], a.q_in[3 * o + 2]);
@@ -1175,7 +1177,7 @@ __global__ void commit_kernel(float4* pos, const float4* prev, const float4* dis
 }
 
 struct FinalizeArgs {
-    const int* perm;
+    const int* inv_perm;
     const float4* pos;
     const float4* prev;
     float* q_in;
@@ -1190,10 +1192,12 @@ struct FinalizeArgs {
     float dt;
 };
 
+// a thread per particle in model order: the caller's arrays are written coalesced, and the internal
+// ones are read in runs (consecutive particles alternate between few colors)
 __global__ void finalize_kernel(FinalizeArgs a) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.V) return;
-    const int o = a.perm[i];
+    const int o = blockIdx.x * blockDim.x + threadIdx.x;
+    if (o >= a.V) return;
+    const int i = a.inv_perm[o];
     const float4 p = a.pos[i], pv = a.prev[i];
     if (a.q_in) {
         a.q_in[3 * o] = p.x;
@@ -1679,7 +1683,7 @@ static void enqueue_finalize(SolverImpl& s, float* q_in, float* q_out, float* qd
                              float* corr = nullptr) {
     const VbdModelImpl& m = *s.m;
     FinalizeArgs a;
-    a.perm = m.perm;
+    a.inv_perm = m.inv_perm;
     a.pinfo = m.pinfo;
     a.y = s.y;
     a.corr = corr;
