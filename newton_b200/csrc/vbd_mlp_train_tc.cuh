@@ -1,11 +1,11 @@
 // vbd_mlp_train_tc.cuh -- loss and parameter gradients of the warm-start MLP (64 -> 128 -> 128 -> 3,
 // SiLU) in one pass over the samples on the 5th-generation tensor cores.  Included by vbd_mlp.cu only.
 //
-// One persistent CTA of 256 threads per SM takes 128-sample tiles.  A tile's activations and their
+// One persistent CTA of 512 threads per SM takes 128-sample tiles.  A tile's activations and their
 // gradients live in shared memory as BF16 operands and never reach HBM; the weight gradients
 // accumulate over all tiles of the CTA in tensor memory (FP32), so that a CTA writes one partial of
 // the parameter blob at its end, and a second kernel adds the partials in CTA order (deterministic).
-// Per tile (thread: one row, half of the 128 columns):
+// Per tile (thread: one row, a quarter of the 128 columns):
 //   Z1 = X W1,  H1 = silu(Z1 + b1);  Z2 = H1 W2,  H2 = silu(Z2 + b2);  Y = H2 W3 + b3, loss, dY
 //   dH2 = dY W3^T,  dZ2 = dH2 silu'(Z2);  dH1 = dZ2 W2^T,  dZ1 = dH1 silu'(Z1)
 //   dW3 += H2^T dY,  dW2 += H1^T dZ2,  dW1^T += dZ1^T X,  db += dZ^T 1  (issued beside the products
@@ -24,8 +24,9 @@
 //
 // What bounds it: two tiles per SM at 32,768 samples, each a serial chain of six products and
 // epilogues; the epilogues' exponentials and reciprocals (4 x 16,384 of each per tile) are the
-// largest part.  Measured at 32,768 samples: 49 us + 8 us for the reduction, against 195 us for the
-// mma.sync passes with their operands in HBM (tile kernel, three split-K products, column sums).
+// largest part, so four warps share a row quarter's columns.  Measured, a training pass over 32,768
+// samples: 45 us with 512 threads (51 with 256), against 195 us for mma.sync passes with their
+// operands in HBM (tile kernel, three split-K products, column sums).
 #pragma once
 
 #include <cuda_bf16.h>
@@ -35,7 +36,8 @@
 namespace vbd {
 namespace tct {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 512;
+constexpr int kCols = 32;  // accumulator columns per thread
 constexpr int kMaxCtas = 148;  // one per SM; partials of the workspace
 constexpr int kRows = 128;
 constexpr int kIn = 64, kHid = 128, kOutP = 8;
@@ -57,7 +59,7 @@ constexpr int kSDZ2 = kSH2 + kRows * kHid * 2;
 constexpr int kSDY = kSDZ2 + kRows * kHid * 2;
 constexpr int kSBias = kSDY + kRows * kN3 * 2;  // b1, b2 [128] and b3 [8] float
 constexpr int kSRed = kSBias + (2 * kHid + kOutP) * 4;  // per-warp sums of loss and db3
-constexpr int kSBar = kSRed + 8 * 4 * 4;
+constexpr int kSBar = kSRed + (kThreads / 32) * 4 * 4;
 constexpr int kSmemBytes = kSBar + 16 + 1024;  // + slack for aligning the base
 
 // tensor memory columns
@@ -122,8 +124,8 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_train_tc_kernel(const __grid_
     uint64_t* bar_slot = reinterpret_cast<uint64_t*>(smem + kSBar);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kSBar + 8);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int quarter = warp & 3, half = warp >> 2;  // TMEM lanes of the warp, its half of the columns
-    const int row = quarter * 32 + lane, c0 = half * 64;
+    const int quarter = warp & 3, part = warp >> 2;  // TMEM lanes of the warp, its quarter of the columns
+    const int row = quarter * 32 + lane, c0 = part * kCols;
 
     // ---- weights [K][N] -> [N][K] operands, ones, biases, mbarrier, TMEM ----
     auto weights = [&](int dst, const uint16_t* src, int K, int N, int R) {
@@ -192,17 +194,17 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_train_tc_kernel(const __grid_
         tc::fence_after();
         return ok;
     };
-    // this thread's half row of BF16 values into a 128-row operand, 8 at a time
+    // this thread's part of a row of BF16 values into a 128-row operand, 8 at a time
     auto store8 = [&](int dst, int c, const unsigned (&w)[4]) {
         *reinterpret_cast<uint4*>(smem + dst + tc::kmajor_offset(row, c, kRows)) = make_uint4(w[0], w[1], w[2], w[3]);
     };
     // X rows of a tile: 8 rows x 64 contiguous bytes per load instruction
-    float4 xv[8];
+    float4 xv[4];
     const bool vec = (reinterpret_cast<uintptr_t>(a.X) & 15u) == 0;
     auto load_x = [&](int tile) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int r = warp * 16 + 8 * (j >> 2) + (lane & 7), c4 = 4 * (j & 3) + (lane >> 3);
+        for (int j = 0; j < 4; ++j) {
+            const int r = warp * 8 + (lane & 7), c4 = 4 * j + (lane >> 3);
             const int s = tile * kRows + r;
             const float* src = a.X + static_cast<size_t>(s) * kIn + 4 * c4;
             xv[j] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -218,13 +220,13 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_train_tc_kernel(const __grid_
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int sample = tile * kRows + row;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int r = warp * 16 + 8 * (j >> 2) + (lane & 7), c4 = 4 * (j & 3) + (lane >> 3);
+        for (int j = 0; j < 4; ++j) {
+            const int r = warp * 8 + (lane & 7), c4 = 4 * j + (lane >> 3);
             *reinterpret_cast<uint2*>(smem + kSX + tc::kmajor_offset(r, 4 * c4, kRows)) =
                 make_uint2(pack2(xv[j].x, xv[j].y), pack2(xv[j].z, xv[j].w));
         }
         float tgt[3] = {0.f, 0.f, 0.f};
-        if (half == 0 && sample < a.n) {
+        if (part == 0 && sample < a.n) {
 #pragma unroll
             for (int c = 0; c < 3; ++c) tgt[c] = __ldg(a.T + static_cast<size_t>(sample) * 3 + c);
         }
@@ -235,12 +237,12 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_train_tc_kernel(const __grid_
             tc::mma_commit(bar);
         }
         if (!await()) break;
-        unsigned z1p[32], z2p[32];  // pre-activations as BF16 pairs, for silu'
-        float acc[64];
-        auto hidden = [&](const float* b, unsigned (&zp)[32], int dst) {
-            tc::tmem_ld64(work + lanes + c0, acc);
+        unsigned z1p[kCols / 2], z2p[kCols / 2];  // pre-activations as BF16 pairs, for silu'
+        float acc[kCols];
+        auto hidden = [&](const float* b, unsigned (&zp)[kCols / 2], int dst) {
+            tc::tmem_ld32(work + lanes + c0, acc);
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
+            for (int q = 0; q < kCols / 8; ++q) {
                 unsigned w[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -266,7 +268,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_train_tc_kernel(const __grid_
             tc::mma_commit(bar);
         }
         if (!await()) break;
-        if (half == 0) {
+        if (part == 0) {
             float y[16];
             tc::tmem_ld16(work + lanes, y);
             float d[3];
@@ -290,10 +292,10 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_train_tc_kernel(const __grid_
             tc::mma_commit(bar);
         }
         if (!await()) break;
-        auto gradient = [&](const unsigned (&zp)[32], int dst) {
-            tc::tmem_ld64(work + lanes + c0, acc);
+        auto gradient = [&](const unsigned (&zp)[kCols / 2], int dst) {
+            tc::tmem_ld32(work + lanes + c0, acc);
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
+            for (int q = 0; q < kCols / 8; ++q) {
                 unsigned w[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -327,21 +329,22 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_train_tc_kernel(const __grid_
     // ---- the CTA's partial of the parameter blob ----
     float* out = a.part + static_cast<size_t>(blockIdx.x) * kPart;
     if (ok) {
-        float acc[64];
-        tc::tmem_ld64(tm + kCW2 + lanes + c0, acc);
+        float acc[kCols];
+        tc::tmem_ld32(tm + kCW2 + lanes + c0, acc);
         float4* o2 = reinterpret_cast<float4*>(out + kOffW2 + row * kHid + c0);
 #pragma unroll
-        for (int q = 0; q < 16; ++q) o2[q] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+        for (int q = 0; q < kCols / 4; ++q) o2[q] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
         float v[16];
-        if (half == 0) {
-            tc::tmem_ld64(tm + kCW1 + lanes, acc);
+        if (part < 2) {  // the inputs' 64 columns
+            tc::tmem_ld32(tm + kCW1 + lanes + c0, acc);
 #pragma unroll
-            for (int f = 0; f < kIn; ++f) out[kOffW1 + f * kHid + row] = acc[f];
-        } else {
+            for (int f = 0; f < kCols; ++f) out[kOffW1 + (c0 + f) * kHid + row] = acc[f];
+        } else if (part == 2) {
             tc::tmem_ld16(tm + kCW3 + lanes, v);
             float4* o3 = reinterpret_cast<float4*>(out + kOffW3 + row * kOutP);
             o3[0] = make_float4(v[0], v[1], v[2], v[3]);
             o3[1] = make_float4(v[4], v[5], v[6], v[7]);
+        } else {
             tc::tmem_ld16(tm + kCB1 + lanes, v);
             out[kOffB1 + row] = v[0];
             tc::tmem_ld16(tm + kCB2 + lanes, v);
@@ -364,7 +367,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_train_tc_kernel(const __grid_
     tc::fence_before();
     __syncthreads();
     if (ok && tid < kOutP) {
-        // half 0's four warps hold the sums
+        // part 0's four warps hold the sums
         auto sum = [&](int k) { return sRed[k] + sRed[4 + k] + sRed[8 + k] + sRed[12 + k]; };
         out[kOffB3 + tid] = tid < 3 ? sum(1 + tid) : 0.f;
         out[kParams + tid] = tid == 0 ? sum(0) : 0.f;
