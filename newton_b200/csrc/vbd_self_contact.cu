@@ -671,8 +671,8 @@ __global__ void tri_sort_kernel(int T, int* tv_count, int* tv_list, int tcap) {
 // Offsets come from scans and every slot from a rank inside a sorted row, so the tables do not
 // depend on thread scheduling.  Rows that would end beyond a table's capacity are left out of it
 // and evaluated from the detection lists.
-constexpr long long kEntriesPerVertex = 128;  // capacities, per vertex on average
-constexpr long long kPairsPerVertex = 32;
+constexpr long long kEntriesPerVertex = 96;   // capacities, per vertex on average (51 and 13 in the case above)
+constexpr long long kPairsPerVertex = 24;
 constexpr int kIdMask = 0x3fffffff;           // vertex ids are below 2^30
 
 __device__ __forceinline__ int tag(int id, int bits) {
@@ -1493,20 +1493,29 @@ int self_contact_create(const VbdModelImpl& m, const SelfContactParams& p, SelfC
         placed.emplace_back(ptr, total);
         total += (std::max<size_t>(bytes, 16) + 255) & ~static_cast<size_t>(255);
     };
+    // what a detection clears, in one span (cleared_bytes): counts, cursors, and the contact terms of
+    // vertices that touch no pair, which stay zero until the next one
     az(reinterpret_cast<void**>(&sc.tri_cnt), tn * sizeof(int));
-    az(reinterpret_cast<void**>(&sc.tri_off), tn * sizeof(int));
     az(reinterpret_cast<void**>(&sc.tri_cur), tn * sizeof(int));
-    az(reinterpret_cast<void**>(&sc.tri_items), static_cast<size_t>(sc.tri_items_cap) * sizeof(int));
     az(reinterpret_cast<void**>(&sc.edge_cnt), en * sizeof(int));
-    az(reinterpret_cast<void**>(&sc.edge_off), en * sizeof(int));
     az(reinterpret_cast<void**>(&sc.edge_cur), en * sizeof(int));
+    az(reinterpret_cast<void**>(&sc.tv_count), static_cast<size_t>(T) * sizeof(int));
+    az(reinterpret_cast<void**>(&sc.vt_count), static_cast<size_t>(V) * sizeof(int));
+    az(reinterpret_cast<void**>(&sc.ee_count), static_cast<size_t>(E) * sizeof(int));
+    az(reinterpret_cast<void**>(&sc.act_vcnt), static_cast<size_t>(std::max(m.C, 1)) * sizeof(int));
+    az(reinterpret_cast<void**>(&sc.sc_f), static_cast<size_t>(V) * sizeof(float4));
+    az(reinterpret_cast<void**>(&sc.sc_h0), static_cast<size_t>(V) * sizeof(float4));
+    az(reinterpret_cast<void**>(&sc.sc_h1), static_cast<size_t>(V) * sizeof(float4));
+    sc.cleared_bytes = total;
+    az(reinterpret_cast<void**>(&sc.tri_off), tn * sizeof(int));
+    az(reinterpret_cast<void**>(&sc.tri_items), static_cast<size_t>(sc.tri_items_cap) * sizeof(int));
+    az(reinterpret_cast<void**>(&sc.edge_off), en * sizeof(int));
     az(reinterpret_cast<void**>(&sc.edge_items), static_cast<size_t>(sc.edge_items_cap) * sizeof(int));
     az(reinterpret_cast<void**>(&sc.tri_box), 2 * static_cast<size_t>(std::max(T, 1)) * sizeof(float4));
     az(reinterpret_cast<void**>(&sc.edge_box), 2 * static_cast<size_t>(std::max(E, 1)) * sizeof(float4));
     az(reinterpret_cast<void**>(&sc.tri_item_box), 2 * static_cast<size_t>(sc.tri_items_cap) * sizeof(float4));
     az(reinterpret_cast<void**>(&sc.edge_item_box), 2 * static_cast<size_t>(sc.edge_items_cap) * sizeof(float4));
     az(reinterpret_cast<void**>(&sc.act_v), static_cast<size_t>(V) * sizeof(int));
-    az(reinterpret_cast<void**>(&sc.act_vcnt), static_cast<size_t>(std::max(m.C, 1)) * sizeof(int));
     const size_t rows = static_cast<size_t>(V) + E + 1;
     sc.ent_cap = kEntriesPerVertex * V;
     sc.pair_cap = kPairsPerVertex * V;
@@ -1518,17 +1527,11 @@ int self_contact_create(const VbdModelImpl& m, const SelfContactParams& p, SelfC
     az(reinterpret_cast<void**>(&sc.pair_ids), static_cast<size_t>(sc.pair_cap) * sizeof(int4));
     az(reinterpret_cast<void**>(&sc.pair_n), static_cast<size_t>(sc.pair_cap) * sizeof(float4));
     az(reinterpret_cast<void**>(&sc.pair_h), static_cast<size_t>(sc.pair_cap) * sizeof(float4));
-    az(reinterpret_cast<void**>(&sc.vt_count), static_cast<size_t>(V) * sizeof(int));
     az(reinterpret_cast<void**>(&sc.vt_list), static_cast<size_t>(V) * p.vertex_buffer * sizeof(int));
-    az(reinterpret_cast<void**>(&sc.ee_count), static_cast<size_t>(E) * sizeof(int));
     az(reinterpret_cast<void**>(&sc.ee_list), static_cast<size_t>(E) * p.edge_buffer * sizeof(int));
-    az(reinterpret_cast<void**>(&sc.tv_count), static_cast<size_t>(T) * sizeof(int));
     az(reinterpret_cast<void**>(&sc.tv_list), static_cast<size_t>(T) * sc.tcap * sizeof(int));
     az(reinterpret_cast<void**>(&sc.cd), static_cast<size_t>(V) * sizeof(float4));
     az(reinterpret_cast<void**>(&sc.reach), static_cast<size_t>(V));
-    az(reinterpret_cast<void**>(&sc.sc_f), static_cast<size_t>(V) * sizeof(float4));
-    az(reinterpret_cast<void**>(&sc.sc_h0), static_cast<size_t>(V) * sizeof(float4));
-    az(reinterpret_cast<void**>(&sc.sc_h1), static_cast<size_t>(V) * sizeof(float4));
     az(reinterpret_cast<void**>(&sc.ts), static_cast<size_t>(V) * sizeof(unsigned));
     az(reinterpret_cast<void**>(&sc.counters), kScCounters * sizeof(unsigned));
     if (!rc) {
@@ -1585,11 +1588,7 @@ int self_contact_detect(const VbdModelImpl& m, SelfContact& sc, const float4* po
                                                            1.0f / sc.reach_unit);
     VBD_CUDA_TRY(cudaGetLastError());
     const unsigned tn = sc.tri_mask + 1, en = sc.edge_mask + 1;
-    VBD_CUDA_TRY(cudaMemsetAsync(sc.tri_cnt, 0, tn * sizeof(int), st));
-    VBD_CUDA_TRY(cudaMemsetAsync(sc.tri_cur, 0, tn * sizeof(int), st));
-    VBD_CUDA_TRY(cudaMemsetAsync(sc.edge_cnt, 0, en * sizeof(int), st));
-    VBD_CUDA_TRY(cudaMemsetAsync(sc.edge_cur, 0, en * sizeof(int), st));
-    if (T > 0) VBD_CUDA_TRY(cudaMemsetAsync(sc.tv_count, 0, static_cast<size_t>(T) * sizeof(int), st));
+    VBD_CUDA_TRY(cudaMemsetAsync(sc.arena, 0, sc.cleared_bytes, st));
     const float inv_cell = 1.0f / sc.cell;
     GridArgs g;
     g.x = sc.cd;
@@ -1682,7 +1681,6 @@ int self_contact_detect(const VbdModelImpl& m, SelfContact& sc, const float4* po
         const long long threads = static_cast<long long>(rows) * kSortLanes;
         sort_rows_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, st>>>(rows, count, list, buf, overflow);
     };
-    VBD_CUDA_TRY(cudaMemsetAsync(sc.vt_count, 0, static_cast<size_t>(V) * sizeof(int), st));
     if (T > 0) {
         const long long vt_threads = static_cast<long long>(V) * kVtLanes;
         vt_query_kernel<<<static_cast<unsigned>((vt_threads + kQueryBlock - 1) / kQueryBlock), kQueryBlock, 0, st>>>(q);
@@ -1696,18 +1694,12 @@ int self_contact_detect(const VbdModelImpl& m, SelfContact& sc, const float4* po
         VBD_CUDA_TRY(cudaGetLastError());
     }
     if (E > 0) {
-        VBD_CUDA_TRY(cudaMemsetAsync(sc.ee_count, 0, static_cast<size_t>(E) * sizeof(int), st));
         const long long ee_threads = static_cast<long long>(E) * kEeLanes;
         ee_query_kernel<<<static_cast<unsigned>((ee_threads + kQueryBlock - 1) / kQueryBlock), kQueryBlock, 0, st>>>(q);
         VBD_CUDA_TRY(cudaGetLastError());
         sort_rows(E, sc.ee_count, sc.ee_list, sc.p.edge_buffer, nullptr);
         VBD_CUDA_TRY(cudaGetLastError());
     }
-    // vertices that touch no pair keep a zero contact term until the next detection
-    VBD_CUDA_TRY(cudaMemsetAsync(sc.sc_f, 0, static_cast<size_t>(V) * sizeof(float4), st));
-    VBD_CUDA_TRY(cudaMemsetAsync(sc.sc_h0, 0, static_cast<size_t>(V) * sizeof(float4), st));
-    VBD_CUDA_TRY(cudaMemsetAsync(sc.sc_h1, 0, static_cast<size_t>(V) * sizeof(float4), st));
-    VBD_CUDA_TRY(cudaMemsetAsync(sc.act_vcnt, 0, static_cast<size_t>(std::max(sc.C, 1)) * sizeof(int), st));
     TableArgs t;
     t.V = V;
     t.E = E;

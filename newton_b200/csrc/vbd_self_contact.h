@@ -59,6 +59,7 @@ struct SelfContact {
     unsigned tri_mask = 0, edge_mask = 0;
     int tri_items_cap = 0, edge_items_cap = 0;
     unsigned char* arena = nullptr;  // every scratch array below is a part of it
+    size_t cleared_bytes = 0;        // its first part, cleared by every detection
     // topology, internal vertex ids
     int4* tri = nullptr;     // [T] a, b, c, world of a
     int4* edge = nullptr;    // [E] v0, v1, world of v0, 0

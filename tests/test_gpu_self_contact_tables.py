@@ -60,10 +60,10 @@ def test_tables_within_and_beyond_their_capacity(margin, beyond):
     np.testing.assert_array_equal(vl, ovl)
     np.testing.assert_array_equal(ec, oec)
     np.testing.assert_array_equal(el, oel)
-    # the capacities are 128 entries and 32 pairs per vertex on average; a pair has four entries
+    # the capacities are 96 entries and 24 pairs per vertex on average; a pair has four entries
     V = model.particle_count
     pairs = int(vc.sum()) + int(ec.sum()) // 2
-    assert (pairs > 32 * V) == beyond and (4 * pairs > 128 * V) == beyond
+    assert (pairs > 24 * V) == beyond and (4 * pairs > 96 * V) == beyond
     exact = oracle.VBDOracle(model, "f64")
     exact.set_self_contact(radius=RADIUS, margin=margin, vertex_buffer=BUFFERS[0], edge_buffer=BUFFERS[1],
                            rest_q=model.particle_q)
