@@ -179,7 +179,9 @@ __device__ __forceinline__ float3 project_cross(float inv_len, float3 nh, float3
     return cross(p, u);
 }
 
-// unit normals n1h, n2h, unit hinge eh, their inverse lengths, and the angle; false: degenerate
+// unit normals n1h, n2h, unit hinge eh, their inverse lengths, and the angle; false: degenerate (the
+// values are then of no use; formed all the same, so that no branch keeps a caller from overlapping
+// this with independent work)
 struct Hinge {
     float3 n1h, n2h, eh;
     float i1, i2, sin_t, cos_t, theta;
@@ -191,7 +193,6 @@ __device__ __forceinline__ bool hinge_set(float3 x02, float3 x03, float3 x13, fl
     const float3 n2 = cross(x13, x12);
     // |n| < eps  <=>  |n|^2 < eps^2; the unit vectors use the hardware reciprocal square root
     const float d1 = dot(n1, n1), d2 = dot(n2, n2), de = dot(e, e);
-    if (d1 < eps * eps || d2 < eps * eps || de < eps * eps) return false;
     g.i1 = rsqrtf(d1);
     g.i2 = rsqrtf(d2);
     g.n1h = n1 * g.i1;
@@ -200,7 +201,7 @@ __device__ __forceinline__ bool hinge_set(float3 x02, float3 x03, float3 x13, fl
     g.sin_t = dot(cross(g.n1h, g.n2h), g.eh);
     g.cos_t = dot(g.n1h, g.n2h);
     g.theta = atan2_as(g.sin_t, g.cos_t);
-    return true;
+    return !(d1 < eps * eps || d2 < eps * eps || de < eps * eps);
 }
 
 // the hinge's angle at the step's start (kNoAngle: degenerate), for damping: once per step
@@ -222,7 +223,7 @@ __device__ __forceinline__ void bending_eval(int order, float3 x0, float3 x1, fl
     const float3 x12 = x2 - x1;
     const float3 e = x3 - x2;
     Hinge q;
-    if (!hinge_set(x02, x03, x13, x12, e, q)) return;
+    const bool ok = hinge_set(x02, x03, x13, x12, e, q);
     const float dE = k * (q.theta - rest);
 
     // Selected dtheta/dx (see header comment):
@@ -236,6 +237,7 @@ __device__ __forceinline__ void bending_eval(int order, float3 x0, float3 x1, fl
     const float3 t2 = project_cross(q.i2, q.n2h, y2, u2);
     const float3 d12 = t1 - t2;
     const float3 g = order == 0 ? t1 : (order == 1 ? -t2 : (order == 2 ? -d12 : d12));
+    if (!ok) return;
     f = f + (-dE) * g;
     add_outer(h, k, g);
 

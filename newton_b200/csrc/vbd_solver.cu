@@ -583,12 +583,40 @@ __device__ __forceinline__ void add_hinge(const SweepArgs& a, const HingeRecord&
 // record's loads and math overlaps the other's.  Used where the launch leaves registers for it (few
 // lanes per vertex, uncapped build).  A lane with an odd count evaluates its last record twice and
 // keeps one result.
-template <int kDamp, bool kStaged, bool kTwo, bool kBulk>
+// kPair (16 lanes, where a lane has one or two records and a launch is one latency chain): the
+// lane's first triangle and its first hinge likewise as two independent chains.  10 iterations, one
+// chain after the other against both together: hanging cloth of 32^2 148 -> 134 us, 64^2 168 -> 158,
+// 124^2 197 -> 191; damped curtain of 64^2 138 -> 127, 120^2 164 -> 165.  At 8 lanes it gave 0.6% and
+// cost the gate's sweep 7% (its registers: two color grids no longer fit an SM together).
+enum Walk { kSingle = 0, kTwo = 1, kPair = 2 };
+
+template <int kDamp, bool kStaged, int kWalk, bool kBulk>
 __device__ __forceinline__ void accumulate_elements(const SweepArgs& a, int lane, int L, int4 adj, const float4* s_pos,
                                                     const BulkRecords* bulk, float3& f, Sym3& h) {
     const int nt = adj.y - adj.x;
     const int lane_e = (lane - nt % L + L) % L;  // first hinge slot of this lane
-    if (!kTwo) {
+    if (kWalk == kPair && nt > 0 && adj.w > adj.z) {
+        const int rt = adj.x + lane, rh = adj.z + lane_e;
+        const bool tri = rt < adj.y, hinge = rh < adj.w;
+        const TriRecord ta = load_tri<kDamp, kStaged>(a, tri ? rt : adj.x, s_pos);
+        const HingeRecord tb = load_hinge<kDamp, kStaged>(a, hinge ? rh : adj.z, s_pos);
+        float3 fa = f3(0.f, 0.f, 0.f), fb = fa;
+        Sym3 ha = zero_sym(), hb = zero_sym();
+        add_hinge<kDamp>(a, tb, fb, hb);
+        add_tri<kDamp>(a, ta, fa, ha);
+        if (tri) {
+            f = f + fa;
+            add(h, ha);
+        }
+        for (int r = rt + L; r < adj.y; r += L) add_tri<kDamp>(a, load_tri<kDamp, kStaged>(a, r, s_pos), f, h);
+        if (hinge) {
+            f = f + fb;
+            add(h, hb);
+        }
+        for (int r = rh + L; r < adj.w; r += L) add_hinge<kDamp>(a, load_hinge<kDamp, kStaged>(a, r, s_pos), f, h);
+        return;
+    }
+    if (kWalk != kTwo) {
         for (int r = adj.x + lane; r < adj.y; r += L)
             add_tri<kDamp>(a, load_tri<kDamp, kStaged, kBulk>(a, r, s_pos, bulk), f, h);
         for (int r = adj.z + lane_e; r < adj.w; r += L)
@@ -926,7 +954,8 @@ __device__ __forceinline__ void sweep_body(const SweepArgs& a) {
     if (valid && solve) {
         BulkRecords bulk = {};
         if (kBulk) bulk = bulk_records(a, vb);
-        accumulate_elements<kDamp, kStaged, (L <= 2 && !kCap), kBulk>(a, lane, L, adj, s_pos, &bulk, f, h);
+        constexpr int kWalk = kCap ? kSingle : (L <= 2 ? kTwo : (L == 16 ? kPair : kSingle));
+        accumulate_elements<kDamp, kStaged, kWalk, kBulk>(a, lane, L, adj, s_pos, &bulk, f, h);
     }
     if (L > 1) {
         f.x = warp_sum(f.x, L);
@@ -1002,8 +1031,11 @@ __global__ void __launch_bounds__(256, kCap ? 4 : 1) sweep_kernel(SweepArgs a) {
 // plain sweep: at 74 (what the compiler picks for the extra reduction) the allocation rounds up
 // to 80 registers per thread, two color grids no longer fit on an SM together, and each launch
 // loses its overlap with the previous one.
+// (16 lanes: small grids, and the pair walk needs more.)
+constexpr int sweep_registers(int L) { return L == 16 ? 112 : 72; }
+
 template <int L, int kDamp, bool kStaged = false>
-__global__ void __maxnreg__(72) sweep_gate_kernel(SweepArgs a) {
+__global__ void __maxnreg__(sweep_registers(L)) sweep_gate_kernel(SweepArgs a) {
     sweep_body<L, kDamp, false, false, true, kStaged>(a);
 }
 
@@ -1017,7 +1049,7 @@ __global__ void __maxnreg__(kCap ? 64 : 72) sweep_bulk_kernel(SweepArgs a) {
 // The staged sweep at 4 or more lanes, held to the same 72 registers (unbounded, the damping
 // build takes 79).
 template <int L, int kDamp>
-__global__ void __maxnreg__(72) sweep_staged_kernel(SweepArgs a) {
+__global__ void __maxnreg__(sweep_registers(L)) sweep_staged_kernel(SweepArgs a) {
     sweep_body<L, kDamp, false, false, false, true>(a);
 }
 
