@@ -1,7 +1,7 @@
 """Learned warm start for the VBD step.
 
-A per-vertex MLP (64 -> 128 -> 128 -> 3, SiLU; trained with FP32 master weights on BF16 mma.sync
-tiles with FP32 accumulation, run for inference on tcgen05 with FP16 operands and FP32
+A per-vertex MLP (64 -> 128 -> 128 -> 3, SiLU; trained with FP32 master weights on tcgen05 with
+BF16 operands and FP32 accumulation, run for inference on tcgen05 with FP16 operands and FP32
 accumulation) predicts the correction ``x_solved - y`` that the coming step applies to the inertia
 target ``y``, in units of the vertex's characteristic element length, from one-ring features
 (``vbd_mlp_features``).  Two feature sets: ``"corrections"`` (default) -- the inertia offset, the
@@ -18,8 +18,8 @@ The previous correction is a feature and never the start itself: starting from
 the velocity that ``y`` extrapolates), and a trajectory advanced that way gains energy and
 diverges within a few hundred steps on the draped cloth even at 10 iterations.
 
-Everything numeric runs in ``libvbd_b200.so``: features, inference, the backward pass, the
-weight-gradient GEMMs and Adam (``vbd_mlp_*``).  Torch tensors are only the buffers.
+Everything numeric runs in ``libvbd_b200.so``: features, inference, the training pass (loss and
+gradients) and Adam (``vbd_mlp_*``).  Torch tensors are only the buffers.
 """
 
 from __future__ import annotations
