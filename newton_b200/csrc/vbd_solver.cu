@@ -324,7 +324,7 @@ __global__ void prepare_kernel(PrepareArgs a) {
     const int i = tid / kTableLanes, lane = tid % kTableLanes;
     if (i >= a.V) return;
     if (a.tables.tri_c) write_tables(a.tables, i, lane, [&](int j) { return xyz(a.prev[j]); });
-    if (lane == 0) pack_contacts(a, i);
+    if (lane == 0 && a.ctab) pack_contacts(a, i);
 }
 
 // What a residual check needs besides the state (baked into the step graph).
@@ -1611,6 +1611,26 @@ static void launch_sweep(const SweepArgs& a, int lanes, int damp, bool residual,
     }
 }
 
+static StepTables step_tables(const SolverImpl& s) {
+    const VbdModelImpl& m = *s.m;
+    return {m.vadj, m.tri_idx, m.tri_D, m.edge_idx, m.edge_kd, s.tri_c, s.edge_th};
+}
+
+// Before a sweep outside a step.  A resident step damps from the step-start positions and leaves the
+// tables as they were, so a solver that can run one has them written here, from those positions.
+static int refresh_tables(SolverImpl& s, cudaStream_t st) {
+    if (!s.tri_c || !s.resident.ready || s.m->V == 0) return VBD_OK;
+    PrepareArgs p;
+    std::memset(&p, 0, sizeof(p));
+    p.prev = s.prev;
+    p.tables = step_tables(s);
+    p.V = s.m->V;
+    const long long threads = static_cast<long long>(p.V) * kTableLanes;
+    prepare_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, st>>>(p);
+    VBD_CUDA_TRY(cudaGetLastError());
+    return VBD_OK;
+}
+
 static int enqueue_forward(SolverImpl& s, const float* q_in, const float* qd_in, const float* f_ext,
                            const VbdContacts* c, float dt, cudaStream_t st, bool tables = true) {
     const VbdModelImpl& m = *s.m;
@@ -1648,7 +1668,7 @@ static int enqueue_forward(SolverImpl& s, const float* q_in, const float* qd_in,
     const bool pack = a.c_count && s.ctab && m.V > 0;
     StepTables t;
     std::memset(&t, 0, sizeof(t));
-    if (tables && s.tri_c) t = {m.vadj, m.tri_idx, m.tri_D, m.edge_idx, m.edge_kd, s.tri_c, s.edge_th};
+    if (tables && s.tri_c) t = step_tables(s);
     if (!pack) a.tables = t;
     const int block = 256;
     const long long threads = static_cast<long long>(m.V) * kTableLanes;
@@ -2445,6 +2465,8 @@ extern "C" int vbd_sweep_color(VbdSolver* solver, int32_t color, const VbdContac
     if (color < 0 || color >= s.m->C) return fail(VBD_ERR_INVALID_ARGUMENT, "vbd_sweep_color: color out of range");
     if (!(dt > 0.0f)) return fail(VBD_ERR_INVALID_ARGUMENT, "vbd_sweep_color: dt must be > 0");
     if (contacts && !contacts->soft_contact_count) contacts = nullptr;
+    const int rc = refresh_tables(s, static_cast<cudaStream_t>(stream));
+    if (rc) return rc;
     enqueue_color(s, color, contacts, dt, static_cast<cudaStream_t>(stream), s.staged_iteration == 0);
     VBD_CUDA_TRY(cudaGetLastError());
     return VBD_OK;
@@ -2575,6 +2597,8 @@ extern "C" int vbd_residual(VbdSolver* solver, const VbdContacts* contacts, floa
     const VbdModelImpl& m = *s.m;
     if (contacts && !contacts->soft_contact_count) contacts = nullptr;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int rt = refresh_tables(s, st);
+    if (rt) return rt;
     float* mx = max_out ? max_out : s.resid_max;
     VBD_CUDA_TRY(cudaMemsetAsync(mx, 0, sizeof(float), st));
     if (per_vertex_out && m.V > m.swept) VBD_CUDA_TRY(cudaMemsetAsync(per_vertex_out, 0, sizeof(float) * m.V, st));
