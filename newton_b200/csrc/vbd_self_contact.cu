@@ -901,19 +901,26 @@ __global__ void table_entries_kernel(const __grid_constant__ TableArgs a) {
     }
 }
 
-// base positions of a detection; the displacements from them are reset, or (the step's start) given
+// base positions of a detection; the displacements from them are reset, or (the step's start) given, or
+// not known (disp NULL: the iterate has nothing to do with the detected positions, no bound holds)
 __global__ void copy_positions_kernel(int V, const float4* src, float4* cd, float4* disp, bool reset,
                                       unsigned char* reach, float reach_inv) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= V) return;
     if (src != cd) cd[i] = src[i];
     if (disp && reset) disp[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    reach[i] = (disp && !reset) ? reach_of(length(xyz(disp[i])), reach_inv) : 0;
+    reach[i] = static_cast<unsigned char>(!disp ? kReachUnbounded
+                                                : (reset ? 0 : reach_of(length(xyz(disp[i])), reach_inv)));
 }
 
-__global__ void refresh_reach_kernel(int V, const float4* disp, unsigned char* reach, float reach_inv) {
+// (a position that is not its base plus its displacement: no bound holds)
+__global__ void refresh_reach_kernel(int V, const float4* cd, const float4* pos, const float4* disp,
+                                     unsigned char* reach, float reach_inv) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < V) reach[i] = reach_of(length(xyz(disp[i])), reach_inv);
+    if (i >= V) return;
+    const float4 c = cd[i], x = pos[i], d = disp[i];
+    const bool moved = x.x == __fadd_rn(c.x, d.x) && x.y == __fadd_rn(c.y, d.y) && x.z == __fadd_rn(c.z, d.z);
+    reach[i] = static_cast<unsigned char>(moved ? reach_of(length(xyz(d)), reach_inv) : kReachUnbounded);
 }
 
 __global__ void load_positions_kernel(int V, const int* perm, const float* q, float4* cd) {
@@ -1573,9 +1580,10 @@ int self_contact_load_positions(const VbdModelImpl& m, SelfContact& sc, const fl
     return VBD_OK;
 }
 
-int self_contact_refresh_reach(const VbdModelImpl& m, SelfContact& sc, const float4* disp, cudaStream_t st) {
+int self_contact_refresh_reach(const VbdModelImpl& m, SelfContact& sc, const float4* pos, const float4* disp,
+                               cudaStream_t st) {
     if (m.V == 0) return VBD_OK;
-    refresh_reach_kernel<<<(m.V + 255) / 256, 256, 0, st>>>(m.V, disp, sc.reach, 1.0f / sc.reach_unit);
+    refresh_reach_kernel<<<(m.V + 255) / 256, 256, 0, st>>>(m.V, sc.cd, pos, disp, sc.reach, 1.0f / sc.reach_unit);
     VBD_CUDA_TRY(cudaGetLastError());
     return VBD_OK;
 }

@@ -51,8 +51,8 @@ struct SelfContact {
     int V = 0, T = 0, E = 0;
     float cell = 0.f;       // grid cell edge
     float max_disp = 0.f;   // margin * relaxation * 0.5
-    // [V] |displacement from cd| of each vertex in units of reach_unit, rounded up (kReachUnbounded:
-    // beyond the range): an upper bound a byte wide, for the force pass's early rejection
+    // [V] |iterate - cd| of each vertex in units of reach_unit, rounded up (kReachUnbounded: beyond the
+    // range, or not known): an upper bound a byte wide, for the force pass's early rejection
     unsigned char* reach = nullptr;
     float reach_unit = 0.f;
     int tcap = 32;          // colliding vertices kept per triangle
@@ -114,7 +114,8 @@ struct SelfContact {
 
 int self_contact_create(const VbdModelImpl& m, const SelfContactParams& p, SelfContact& sc);
 void self_contact_free(SelfContact& sc);
-// Detection at `positions` (internal order): cd := positions, and disp := 0 when reset_disp.
+// Detection at `positions` (internal order): cd := positions, and disp := 0 when reset_disp.  disp NULL:
+// positions of their own, which the iterate is not a displacement of.
 int self_contact_detect(const VbdModelImpl& m, SelfContact& sc, const float4* positions, float4* disp,
                         bool reset_disp, cudaStream_t st);
 // Force / Hessian of every pair of the contact-touching vertices of `color` (-1: all colors)
@@ -125,8 +126,9 @@ int self_contact_accumulate(const VbdModelImpl& m, SelfContact& sc, const float4
 // changed: those of `color` (-1: every vertex) and those that a plane shortens.
 int self_contact_truncate(const VbdModelImpl& m, SelfContact& sc, float4* pos, float4* disp, int color,
                           cudaStream_t st);
-// The byte bounds of all displacements (after something else than a sweep changed them).
-int self_contact_refresh_reach(const VbdModelImpl& m, SelfContact& sc, const float4* disp, cudaStream_t st);
+// The byte bounds of all displacements (after something else than a sweep moved the iterate).
+int self_contact_refresh_reach(const VbdModelImpl& m, SelfContact& sc, const float4* pos, const float4* disp,
+                               cudaStream_t st);
 // Whether iteration `it` begins with a detection (particle_collision_detection_interval).
 bool self_contact_detect_now(const SelfContact& sc, int it);
 // Loads model-order positions [V,3] into cd (internal order) -- for detection from a given state.

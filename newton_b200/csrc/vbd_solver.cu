@@ -2487,7 +2487,7 @@ extern "C" int vbd_warm_start(VbdSolver* solver, const float* delta, void* strea
     warm_start_kernel<<<(s.m->V + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(
         s.m->perm, s.m->pinfo, s.prev, s.disp, s.pos, delta, s.m->V);
     VBD_CUDA_TRY(cudaGetLastError());
-    if (s.sc.on) return self_contact_refresh_reach(*s.m, s.sc, s.disp, static_cast<cudaStream_t>(stream));
+    if (s.sc.on) return self_contact_refresh_reach(*s.m, s.sc, s.pos, s.disp, static_cast<cudaStream_t>(stream));
     return VBD_OK;
 }
 

@@ -1,0 +1,92 @@
+"""The early rejection of the self-contact force pass (a pair's distance at the detected positions less
+what its vertices have moved since) never changes a result: the forces equal, bit for bit, those of the
+same detection without displacement bounds (``self_contact_detect`` gives the pass none)."""
+
+import numpy as np
+import pytest
+import torch
+
+from newton_b200 import ModelBuilder, scenes
+from newton_b200.solvers import SolverVBD
+
+pytestmark = pytest.mark.gpu
+DT = 1.0 / 600.0
+
+
+def _layers(n, cell, gap, shift=0.0):
+    """Two square cloths of n x n vertices, the upper one turned by 90 degrees, shifted and lifted by gap."""
+    b = ModelBuilder()
+    verts, tris = ModelBuilder.grid_mesh(n - 1, n - 1, cell, cell)
+    for k in range(2):
+        b.add_cloth_mesh(pos=(0.0, 0.0, 0.0), rot=(0.0, 0.0, 0.0, 1.0), scale=1.0, vel=(0.0, 0.0, 0.0), vertices=verts,
+                         indices=tris, density=0.1, tri_ke=1.0e3, tri_ka=1.0e3, tri_kd=0.0, edge_ke=0.0, edge_kd=0.0)
+    b.color()
+    model = b.finalize()
+    model.soft_contact_ke, model.soft_contact_kd, model.soft_contact_mu = 1.0e3, 1.0e-2, 0.2
+    q = model.particle_q.astype(np.float64).copy()
+    side = cell * (n - 1)
+    up = np.arange(q.shape[0]) >= n * n
+    x, y = q[up, 0].copy(), q[up, 1].copy()
+    q[up, 0], q[up, 1] = side - y + shift, x + shift
+    q[up, 2] += gap
+    return model, q.astype(np.float32), up
+
+
+def _residuals(model, q, qd, radius, margin):
+    """(after forward, after detecting again at the step's start, after detecting at the iterate)"""
+    solver = SolverVBD(model, iterations=1, particle_enable_self_contact=True, particle_self_contact_radius=radius,
+                       particle_self_contact_margin=margin, particle_vertex_contact_buffer_size=128,
+                       particle_edge_contact_buffer_size=256)
+    state = model.state()
+    state.particle_q.copy_(torch.from_numpy(q).cuda())
+    state.particle_qd.copy_(torch.from_numpy(qd).cuda())
+    solver.forward(state, None, DT)
+    moved = solver.positions()
+    out = [solver.residual(None, DT, per_vertex=True)[1].cpu().numpy()]
+    for at in (state.particle_q, moved):
+        solver.self_contact_detect(at)
+        out.append(solver.residual(None, DT, per_vertex=True)[1].cpu().numpy())
+    assert solver.status()["self_contact_overflow"] == 0
+    return out
+
+
+def test_detection_at_other_positions_than_the_iterate():
+    """The layers are 3 mm apart at the step's start (radius 2 mm) and 1.5 mm apart at the iterate: the
+    forces are the same whether the pairs were detected at the former or at the latter."""
+    model, q, up = _layers(12, 0.02, 0.003, 0.006)
+    qd = np.zeros_like(q)
+    qd[up, 2] = -0.0015 / DT
+    first, again, there = _residuals(model, q, qd, 0.002, 0.004)
+    solo, _, _ = _residuals(model, q + np.where(up, 0.1, 0.0)[:, None].astype(np.float32), qd, 0.002, 0.004)
+    assert np.abs(first - solo).max() > 1e3 * np.abs(solo).max()  # (contact forces are there)
+    np.testing.assert_array_equal(first, again)
+    # other lists, other order of the same FP32 sums
+    np.testing.assert_allclose(again, there, rtol=1e-4, atol=1e-5 * there.max())
+
+
+def test_warm_start_from_another_base_than_the_detected_one():
+    """``warm_start`` puts the iterate at the step's start (3 mm apart, radius 3.2 mm) plus its displacement,
+    after a detection at the iterate (4 mm apart) that made those positions the base."""
+    model, q, up = _layers(12, 0.02, 0.003, 0.006)
+    qd = np.zeros_like(q)
+    qd[up, 2] = 0.001 / DT
+
+    def residuals(q):
+        solver = SolverVBD(model, iterations=1, particle_enable_self_contact=True, particle_self_contact_radius=0.0032,
+                           particle_self_contact_margin=0.005)
+        state = model.state()
+        state.particle_q.copy_(torch.from_numpy(q).cuda())
+        state.particle_qd.copy_(torch.from_numpy(qd).cuda())
+        solver.forward(state, None, DT)
+        base = solver.positions()
+        solver.begin_iteration()
+        solver.warm_start(torch.zeros_like(state.particle_q))
+        assert torch.equal(solver.positions(), state.particle_q)
+        first = solver.residual(None, DT, per_vertex=True)[1].cpu().numpy()
+        solver.self_contact_detect(base)
+        return first, solver.residual(None, DT, per_vertex=True)[1].cpu().numpy()
+
+    first, again = residuals(q)
+    solo, _ = residuals(q + np.where(up, 0.1, 0.0)[:, None].astype(np.float32))
+    assert np.abs(first - solo).max() > 2.0 * np.abs(solo).max()  # (contact forces are there)
+    np.testing.assert_array_equal(first, again)
