@@ -214,17 +214,25 @@ __device__ __forceinline__ float hinge_angle(float3 a0, float3 a1, float3 a2, fl
 // hinges of all four orders, so that branches on the order would run one after the other (the two
 // forms compute the same operations for a given order and give the same bits).  With the damping tables
 // and the area branch, a warp of 8 vertices takes 1,402 instructions per sweep instead of 1,694.
-template <bool kDamping>
-__device__ __forceinline__ void bending_eval(int order, float3 x0, float3 x1, float3 x2, float3 x3, float theta_prev,
-                                             float rest, float k, float kd, float inv_dt, float3& f, Sym3& h) {
+// (In two parts, so that a caller can form a hinge's terms beside other work and add them in their turn.)
+struct BendingTerms {
+    float3 g;  // dtheta / dx of the selected vertex
+    float dE, theta;
+    bool ok;  // false: degenerate, adds nothing
+};
+
+__device__ __forceinline__ BendingTerms bending_terms(int order, float3 x0, float3 x1, float3 x2, float3 x3, float rest,
+                                                      float k) {
     const float3 x02 = x2 - x0;
     const float3 x03 = x3 - x0;
     const float3 x13 = x3 - x1;
     const float3 x12 = x2 - x1;
     const float3 e = x3 - x2;
     Hinge q;
-    const bool ok = hinge_set(x02, x03, x13, x12, e, q);
-    const float dE = k * (q.theta - rest);
+    BendingTerms t;
+    t.ok = hinge_set(x02, x03, x13, x12, e, q);
+    t.dE = k * (q.theta - rest);
+    t.theta = q.theta;
 
     // Selected dtheta/dx (see header comment):
     //   order 0:  T1(y1) x e            order 2:  T2(y2) x x13 - T1(y1) x x03
@@ -236,22 +244,34 @@ __device__ __forceinline__ void bending_eval(int order, float3 x0, float3 x1, fl
     const float3 t1 = project_cross(q.i1, q.n1h, y1, u1);
     const float3 t2 = project_cross(q.i2, q.n2h, y2, u2);
     const float3 d12 = t1 - t2;
-    const float3 g = order == 0 ? t1 : (order == 1 ? -t2 : (order == 2 ? -d12 : d12));
-    if (!ok) return;
-    f = f + (-dE) * g;
-    add_outer(h, k, g);
+    t.g = order == 0 ? t1 : (order == 1 ? -t2 : (order == 2 ? -d12 : d12));
+    return t;
+}
+
+template <bool kDamping>
+__device__ __forceinline__ void bending_add(const BendingTerms& t, float theta_prev, float k, float kd, float inv_dt,
+                                            float3& f, Sym3& h) {
+    if (!t.ok) return;
+    f = f + (-t.dE) * t.g;
+    add_outer(h, k, t.g);
 
     if (kDamping && kd > 0.0f && theta_prev != kNoAngle) {
-        float dth = q.theta - theta_prev;
+        float dth = t.theta - theta_prev;
         if (dth > 3.141592653589793f) {
             dth = dth - 6.283185307179586f;
         } else if (dth < -3.141592653589793f) {
             dth = dth + 6.283185307179586f;
         }
         const float rate = dth * inv_dt;
-        f = f + (-kd * rate) * g;
-        add_outer(h, kd * inv_dt, g);
+        f = f + (-kd * rate) * t.g;
+        add_outer(h, kd * inv_dt, t.g);
     }
+}
+
+template <bool kDamping>
+__device__ __forceinline__ void bending_eval(int order, float3 x0, float3 x1, float3 x2, float3 x3, float theta_prev,
+                                             float rest, float k, float kd, float inv_dt, float3& f, Sym3& h) {
+    bending_add<kDamping>(bending_terms(order, x0, x1, x2, x3, rest, k), theta_prev, k, kd, inv_dt, f, h);
 }
 
 // ---------------------------------------------------------------------------------------------

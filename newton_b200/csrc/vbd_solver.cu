@@ -584,10 +584,13 @@ __device__ __forceinline__ void add_hinge(const SweepArgs& a, const HingeRecord&
 // lanes per vertex, uncapped build).  A lane with an odd count evaluates its last record twice and
 // keeps one result.
 // kPair (16 lanes, where a lane has one or two records and a launch is one latency chain): the
-// lane's first triangle and its first hinge likewise as two independent chains.  10 iterations, one
-// chain after the other against both together: hanging cloth of 32^2 148 -> 134 us, 64^2 168 -> 158,
-// 124^2 197 -> 191; damped curtain of 64^2 138 -> 127, 120^2 164 -> 165.  At 8 lanes it gave 0.6% and
-// cost the gate's sweep 7% (its registers: two color grids no longer fit an SM together).
+// lane's first triangle and its first hinge's terms beside each other, added one after the other as
+// kSingle does, so that both give the same bits (which of them runs depends on a build's occupancy, and
+// staged, gated and plain sweeps must agree).  10 iterations, one chain after the other against both
+// together: hanging cloth of 32^2 148 -> 134 us, 64^2 168 -> 158, 124^2 197 -> 191; damped curtain of
+// 64^2 138 -> 127, 120^2 164 -> 165 (with two separate sums; in this form a step is another 1 to 3%
+// shorter: hanging 64^2 117.3 -> 115.4, curtain 120^2 162.4 -> 157.7 for the step alone).  At 8 lanes it
+// gave 0.6% and cost the gate's sweep 7% (its registers: two color grids no longer fit an SM together).
 enum Walk { kSingle = 0, kTwo = 1, kPair = 2 };
 
 template <int kDamp, bool kStaged, int kWalk, bool kBulk>
@@ -600,19 +603,16 @@ __device__ __forceinline__ void accumulate_elements(const SweepArgs& a, int lane
         const bool tri = rt < adj.y, hinge = rh < adj.w;
         const TriRecord ta = load_tri<kDamp, kStaged>(a, tri ? rt : adj.x, s_pos);
         const HingeRecord tb = load_hinge<kDamp, kStaged>(a, hinge ? rh : adj.z, s_pos);
-        float3 fa = f3(0.f, 0.f, 0.f), fb = fa;
-        Sym3 ha = zero_sym(), hb = zero_sym();
-        add_hinge<kDamp>(a, tb, fb, hb);
-        add_tri<kDamp>(a, ta, fa, ha);
+        const BendingTerms b = bending_terms(tb.order, tb.x0, tb.x1, tb.x2, tb.x3, tb.m.x, tb.m.y);
+        float3 ft = f;
+        Sym3 ht = h;
+        add_tri<kDamp>(a, ta, ft, ht);
         if (tri) {
-            f = f + fa;
-            add(h, ha);
+            f = ft;
+            h = ht;
         }
         for (int r = rt + L; r < adj.y; r += L) add_tri<kDamp>(a, load_tri<kDamp, kStaged>(a, r, s_pos), f, h);
-        if (hinge) {
-            f = f + fb;
-            add(h, hb);
-        }
+        if (hinge) bending_add<(kDamp >= kDampAll)>(b, tb.th, tb.m.y, tb.kd, a.inv_dt, f, h);
         for (int r = rh + L; r < adj.w; r += L) add_hinge<kDamp>(a, load_hinge<kDamp, kStaged>(a, r, s_pos), f, h);
         return;
     }
@@ -1447,9 +1447,10 @@ static void launch_staged_LDG(const SweepArgs& a, int grid, int block, cudaStrea
         else
             launch_dependent(sweep_gate_kernel<L, kDamp, true>, grid, block, st, a, smem);
     } else if constexpr (kGate || L <= 2) {
-        // (at 1-2 lanes the two-record walk needs more than 72 registers, as unstaged)
-        const void* uncapped = reinterpret_cast<const void*>(&sweep_kernel<L, kDamp, false, false, kGate, true>);
-        if (grid > resident_blocks(uncapped, block, smem))
+        // (at 1-2 lanes the two-record walk needs more than 72 registers, as unstaged; the two builds
+        // sum in different orders, so the choice is the unstaged sweep's)
+        const void* unstaged = reinterpret_cast<const void*>(&sweep_kernel<L, kDamp, false, false, kGate>);
+        if (grid > resident_blocks(unstaged, block))
             launch_dependent(sweep_kernel<L, kDamp, false, true, kGate, true>, grid, block, st, a, smem);
         else
             launch_dependent(sweep_kernel<L, kDamp, false, false, kGate, true>, grid, block, st, a, smem);
@@ -1467,8 +1468,8 @@ static void prime_staged_occupancy_LD(int block, size_t smem) {
         resident_blocks(reinterpret_cast<const void*>(&sweep_staged_kernel<L, kDamp>), block, smem);
         resident_blocks(reinterpret_cast<const void*>(&sweep_gate_kernel<L, kDamp, true>), block, smem);
     } else {
-        resident_blocks(reinterpret_cast<const void*>(&sweep_kernel<L, kDamp, false, false, false, true>), block, smem);
-        resident_blocks(reinterpret_cast<const void*>(&sweep_kernel<L, kDamp, false, false, true, true>), block, smem);
+        resident_blocks(reinterpret_cast<const void*>(&sweep_kernel<L, kDamp, false, false>), block);
+        resident_blocks(reinterpret_cast<const void*>(&sweep_kernel<L, kDamp, false, false, true>), block);
     }
 }
 
