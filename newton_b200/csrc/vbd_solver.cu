@@ -2314,7 +2314,8 @@ struct Ends {
 constexpr int kConcurrentParticles = 65536;
 
 // Whether the entries of a batch may run beside one another: distinct solvers on one device, small
-// models, and no entry writing what another one reads or writes.
+// models, no resident step (its patches wait for one another and take an SM each, so that two of them
+// may not share the GPU), and no entry writing what another one reads or writes.
 bool batch_independent(VbdSolver* const* solvers, int count, float* const* q_in, const float* const* qd_in,
                        const float* const* f_ext, float* const* q_out, float* const* qd_out,
                        const VbdContacts* const* contacts) {
@@ -2324,8 +2325,10 @@ bool batch_independent(VbdSolver* const* solvers, int count, float* const* q_in,
     std::vector<Access> acc;
     acc.reserve(static_cast<size_t>(count) * 12);
     for (int b = 0; b < count; ++b) {
-        const VbdModelImpl& m = *solvers[b]->s.m;
+        const SolverImpl& s = solvers[b]->s;
+        const VbdModelImpl& m = *s.m;
         if (m.V > kConcurrentParticles || m.device != solvers[0]->s.m->device) return false;
+        if (s.resident_on && s.resident.ready) return false;
         auto add = [&](const void* p, size_t bytes, bool write) {
             const uintptr_t u = reinterpret_cast<uintptr_t>(p);
             if (p && bytes) acc.push_back({u, u + bytes, b, write});

@@ -72,3 +72,23 @@ def test_dependent_entries_run_in_order(twice):
         torch.cuda.synchronize()
         results.append((c.particle_q.clone(), c.particle_qd.clone()))
     assert torch.equal(results[0][0], results[1][0]) and torch.equal(results[0][1], results[1][1])
+
+
+def test_resident_solvers_run_in_order():
+    """A resident step takes one CTA per patch on the whole GPU, its patches waiting for one another, so
+    two of them never run beside each other."""
+    def run(batch):
+        entries = []
+        for k, n in enumerate((64, 96, 80)):
+            model, q0 = scenes.draped_cloth(n=n, seed=k, height=0.902)
+            a, b = model.state(), model.state()
+            a.particle_q.copy_(torch.from_numpy(q0).cuda())
+            pipe = CollisionPipeline(model, soft_contact_margin=5e-3)
+            entries.append([SolverVBD(model, iterations=4, resident_step=k < 2), pipe, pipe.contacts(), a, b])
+        out = _run(entries, 6, batch, torch.cuda.current_stream())
+        for e in entries[:2]:
+            assert e[0].step_kernel_info()["resident"] and e[0].status()["timeouts"] == 0
+        return out
+
+    for (qa, va), (qb, vb) in zip(run(True), run(False)):
+        assert torch.equal(qa, qb) and torch.equal(va, vb)
