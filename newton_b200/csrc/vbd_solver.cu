@@ -1975,6 +1975,8 @@ static int enqueue_step(SolverImpl& s, float* q_in, const float* qd_in, const fl
 // that a block's vertices own.  Off at other lane counts than 4 (fewer lanes: too many records per
 // block; more: too few) and for meshes with runs so long that fewer blocks would fit an SM.
 constexpr int kBulkMaxBytes = 26 * 1024;
+// dynamic shared memory of a launch without opt-in, less the kernel's static part (its mbarrier)
+constexpr int kBulkMaxLaunch = 48 * 1024 - 256;
 
 static void plan_bulk(SolverImpl& s) {
     const VbdModelImpl& m = *s.m;
@@ -1988,7 +1990,8 @@ static void plan_bulk(SolverImpl& s) {
             tri = std::max(tri, last.y - first.x);
             edge = std::max(edge, last.w - first.z);
         }
-    if (tri + edge == 0 || bulk_bytes(tri, edge) * (128.0 / s.block) > kBulkMaxBytes || bulk_bytes(tri, edge) > 48 * 1024)
+    if (tri + edge == 0 || bulk_bytes(tri, edge) * (128.0 / s.block) > kBulkMaxBytes ||
+        bulk_bytes(tri, edge) > kBulkMaxLaunch)
         return;
     s.bulk_tri = tri;
     s.bulk_edge = edge;
