@@ -90,3 +90,42 @@ def test_warm_start_from_another_base_than_the_detected_one():
     solo, _ = residuals(q + np.where(up, 0.1, 0.0)[:, None].astype(np.float32))
     assert np.abs(first - solo).max() > 2.0 * np.abs(solo).max()  # (contact forces are there)
     np.testing.assert_array_equal(first, again)
+
+
+@pytest.mark.parametrize("stretch", [0.04, 0.0, -0.04])
+@pytest.mark.parametrize("cell", [0.0031, 0.0032])
+def test_edges_that_cross_the_length_threshold(cell, stretch):
+    """Edges below sqrt(edge_parallel_epsilon) = 3.16 mm count as points, so stretching one beyond it
+    brings a crossing pair from its first endpoints' distance (2.4 mm) to the crossing's (1 mm)."""
+    model, q, up = _layers(7, cell, 0.001, 0.5 * cell)
+    centre = q.mean(axis=0)
+    qd = (stretch / DT * (q - centre)).astype(np.float32)
+    qd[:, 2] = 0.0
+    first, again, _ = _residuals(model, q, qd, 0.002, 0.003)
+    np.testing.assert_array_equal(first, again)
+
+
+def test_thin_triangles_and_near_parallel_edges():
+    """Random thin cloths (aspect down to 1e-4) across one another, moved at random: where FP32 misses a
+    pair's closest points, its bound must not reject what the direct test takes."""
+    rng = np.random.default_rng(7)
+    model, q, up = _layers(5, 0.004, 0.0025, 0.0)
+    for k in range(12):
+        squeeze = 10.0 ** rng.uniform(-4.0, 0.0)
+        p = q.astype(np.float64).copy()
+        p[:, 1] *= squeeze
+        p[up, 1] += rng.uniform(-1.0, 1.0) * 0.002
+        p = p.astype(np.float32)
+        qd = (rng.uniform(-1.0, 1.0, size=p.shape) * 0.0012 / DT).astype(np.float32)
+        solver = SolverVBD(model, iterations=1, particle_enable_self_contact=True, particle_self_contact_radius=0.002,
+                           particle_self_contact_margin=0.003, particle_vertex_contact_buffer_size=128,
+                           particle_edge_contact_buffer_size=256)
+        state = model.state()
+        state.particle_q.copy_(torch.from_numpy(p).cuda())
+        state.particle_qd.copy_(torch.from_numpy(qd).cuda())
+        solver.forward(state, None, DT)
+        first = solver.residual(None, DT, per_vertex=True)[1].cpu().numpy()
+        solver.self_contact_detect(state.particle_q)
+        again = solver.residual(None, DT, per_vertex=True)[1].cpu().numpy()
+        np.testing.assert_array_equal(first, again)
+        assert solver.status()["self_contact_overflow"] == 0
