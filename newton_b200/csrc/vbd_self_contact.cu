@@ -1264,8 +1264,10 @@ __global__ void __launch_bounds__(kPlanarBlock, kPlanarBlocks) planar_kernel(con
 }
 
 // apply_truncation_ts: disp *= t, clamp |disp| to max_disp, pos = cd + disp; t is reset to 1.  Only
-// where something changed: the vertices [b, e) (the color just solved, or all) and those with t < 1.
-// (The others' displacements and positions already are what the same arithmetic would write.)
+// where that changes something: the vertices [b, e) (the color just solved, or all), those with t < 1, and
+// those without a bound -- displacements beyond max_disp (a warm start's, or one that its clamp left a last
+// place too long; reach_of gives none to either) and positions that are not cd + disp.  The others'
+// displacements and positions already are what the same arithmetic would write.
 __global__ void apply_truncation_kernel(int V, const float4* cd, float4* disp, float4* pos, unsigned* ts,
                                         unsigned char* reach, float reach_inv, float max_disp, int b, int e) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -1273,8 +1275,9 @@ __global__ void apply_truncation_kernel(int V, const float4* cd, float4* disp, f
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= V) return;
     const float t = __uint_as_float(ts[i]);
+    const int bound = reach[i];
     const bool cut = t != 1.0f;
-    if (!cut && (i < b || i >= e)) return;
+    if (!cut && (i < b || i >= e) && bound != kReachUnbounded) return;
     if (cut) ts[i] = __float_as_uint(1.0f);
     const float4 d4 = disp[i];
     float3 d = f3(d4.x * t, d4.y * t, d4.z * t);
@@ -1404,7 +1407,7 @@ int self_contact_create(const VbdModelImpl& m, const SelfContactParams& p, SelfC
     sc.T = T;
     sc.E = E;
     sc.max_disp = static_cast<float>(static_cast<double>(p.margin) * static_cast<double>(p.relaxation) * 0.5);
-    sc.reach_unit = std::max(sc.max_disp, 1e-6f) / 254.0f;
+    sc.reach_unit = std::max(sc.max_disp, 1e-30f) / 254.0f;  // (a displacement beyond max_disp has no bound)
     std::vector<int> inv(V);
     for (int i = 0; i < V; ++i) inv[m.perm_host[i]] = i;
     // topology

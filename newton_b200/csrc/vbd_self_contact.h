@@ -23,7 +23,8 @@ namespace vbd {
 
 constexpr int kReachUnbounded = 255;
 
-// the byte bound of a displacement of length l (NaN: unbounded)
+// the byte bound of a displacement of length l (NaN, or beyond max_disp: unbounded -- the factor rounds
+// lengths from max_disp on past 254)
 __device__ __forceinline__ unsigned char reach_of(float l, float inv_unit) {
     const float u = ceilf(l * inv_unit * 1.0001f);
     return static_cast<unsigned char>(u <= 254.0f ? static_cast<int>(u) : kReachUnbounded);
@@ -123,7 +124,8 @@ int self_contact_detect(const VbdModelImpl& m, SelfContact& sc, const float4* po
 int self_contact_accumulate(const VbdModelImpl& m, SelfContact& sc, const float4* pos, const float4* prev,
                             int color, float dt, float friction_epsilon, cudaStream_t st);
 // Planar truncation of all displacements, then pos := cd + disp for every vertex whose displacement
-// changed: those of `color` (-1: every vertex) and those that a plane shortens.
+// or position changes by it: those of `color` (-1: every vertex), those that a plane shortens and those
+// without a bound in `reach`.
 int self_contact_truncate(const VbdModelImpl& m, SelfContact& sc, float4* pos, float4* disp, int color,
                           cudaStream_t st);
 // The byte bounds of all displacements (after something else than a sweep moved the iterate).

@@ -129,3 +129,23 @@ def test_thin_triangles_and_near_parallel_edges():
         again = solver.residual(None, DT, per_vertex=True)[1].cpu().numpy()
         np.testing.assert_array_equal(first, again)
         assert solver.status()["self_contact_overflow"] == 0
+
+
+def test_warm_start_beyond_the_bound_is_clamped_by_the_first_color():
+    """``warm_start`` may move vertices beyond margin * relaxation / 2; the truncation after the first
+    color brings every vertex back to it, whatever its color."""
+    model, q0 = scenes.single_cloth(n=16, side=1.0, seed=0, pin_top_corners=False, ground=None)
+    margin, bound = 0.004, 0.004 * 0.85 * 0.5
+    solver = SolverVBD(model, iterations=1, particle_enable_self_contact=True, particle_self_contact_radius=0.002,
+                       particle_self_contact_margin=margin, particle_collision_detection_interval=-1)
+    state = model.state()
+    state.particle_q.copy_(torch.from_numpy(q0).cuda())
+    solver.forward(state, None, DT)
+    delta = np.zeros_like(q0)
+    delta[:, 2] = 0.01
+    solver.warm_start(torch.from_numpy(delta).cuda())
+    assert np.linalg.norm(solver.positions().cpu().numpy() - q0, axis=1).min() > bound
+    solver.begin_iteration()
+    solver.sweep_color(0, None, DT)
+    x = solver.positions().cpu().numpy()
+    assert np.linalg.norm(x - q0, axis=1).max() <= bound * (1.0 + 1e-4)
