@@ -671,7 +671,8 @@ __global__ void tri_sort_kernel(int T, int* tv_count, int* tv_list, int tcap) {
 // Offsets come from scans and every slot from a rank inside a sorted row, so the tables do not
 // depend on thread scheduling.  Rows that would end beyond a table's capacity are left out of it
 // and evaluated from the detection lists.
-constexpr long long kEntriesPerVertex = 96;   // capacities, per vertex on average (51 and 13 in the case above)
+// Capacities, per vertex on average (51 and 13 in the case above), where the GPU has the memory: 2,688 bytes.
+constexpr long long kEntriesPerVertex = 96;
 constexpr long long kPairsPerVertex = 24;
 constexpr int kIdMask = 0x3fffffff;           // vertex ids are below 2^30
 
@@ -1346,13 +1347,6 @@ std::vector<int> morton_order(const std::vector<float3>& pts) {
     return order;
 }
 
-int alloc_zero(void** p, size_t bytes) {
-    bytes = std::max<size_t>(bytes, 16);
-    VBD_CUDA_TRY(cudaMalloc(p, bytes));
-    VBD_CUDA_TRY(cudaMemset(*p, 0, bytes));
-    return VBD_OK;
-}
-
 }  // namespace
 
 bool self_contact_detect_now(const SelfContact& sc, int it) {
@@ -1551,16 +1545,10 @@ int self_contact_create(const VbdModelImpl& m, const SelfContactParams& p, SelfC
     az(reinterpret_cast<void**>(&sc.edge_item_box), 2 * static_cast<size_t>(sc.edge_items_cap) * sizeof(float4));
     az(reinterpret_cast<void**>(&sc.act_v), static_cast<size_t>(V) * sizeof(int));
     const size_t rows = static_cast<size_t>(V) + E + 1;
-    sc.ent_cap = kEntriesPerVertex * V;
-    sc.pair_cap = kPairsPerVertex * V;
     az(reinterpret_cast<void**>(&sc.ent_cnt), (static_cast<size_t>(V) + 1) * sizeof(long long));
     az(reinterpret_cast<void**>(&sc.ent_off), (static_cast<size_t>(V) + 1) * sizeof(long long));
-    az(reinterpret_cast<void**>(&sc.ent), static_cast<size_t>(sc.ent_cap) * sizeof(int4));
     az(reinterpret_cast<void**>(&sc.pair_cnt), rows * sizeof(long long));
     az(reinterpret_cast<void**>(&sc.pair_off), rows * sizeof(long long));
-    az(reinterpret_cast<void**>(&sc.pair_ids), static_cast<size_t>(sc.pair_cap) * sizeof(int4));
-    az(reinterpret_cast<void**>(&sc.pair_n), static_cast<size_t>(sc.pair_cap) * sizeof(float4));
-    az(reinterpret_cast<void**>(&sc.pair_h), static_cast<size_t>(sc.pair_cap) * sizeof(float4));
     az(reinterpret_cast<void**>(&sc.vt_list), static_cast<size_t>(V) * p.vertex_buffer * sizeof(int));
     az(reinterpret_cast<void**>(&sc.ee_list), static_cast<size_t>(E) * p.edge_buffer * sizeof(int));
     az(reinterpret_cast<void**>(&sc.tv_list), static_cast<size_t>(T) * sc.tcap * sizeof(int));
@@ -1580,7 +1568,28 @@ int self_contact_create(const VbdModelImpl& m, const SelfContactParams& p, SelfC
         sc.scan_bytes = std::max(std::max(b1, b2), b3);
         az(&sc.scan_tmp, sc.scan_bytes);
     }
-    if (!rc) rc = alloc_zero(reinterpret_cast<void**>(&sc.arena), total);
+    // the pair tables last: where the GPU has no room for them, a quarter, a sixteenth or none of their
+    // capacity (the rows that do not fit are evaluated from the lists)
+    const size_t others = placed.size(), others_bytes = total;
+    for (long long share = 1; !rc && !sc.arena; share *= 4) {
+        placed.resize(others);
+        total = others_bytes;
+        const bool last = share > 16;
+        sc.ent_cap = last ? 0 : kEntriesPerVertex * V / share;
+        sc.pair_cap = last ? 0 : kPairsPerVertex * V / share;
+        az(reinterpret_cast<void**>(&sc.ent), static_cast<size_t>(sc.ent_cap) * sizeof(int4));
+        az(reinterpret_cast<void**>(&sc.pair_ids), static_cast<size_t>(sc.pair_cap) * sizeof(int4));
+        az(reinterpret_cast<void**>(&sc.pair_n), static_cast<size_t>(sc.pair_cap) * sizeof(float4));
+        az(reinterpret_cast<void**>(&sc.pair_h), static_cast<size_t>(sc.pair_cap) * sizeof(float4));
+        cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&sc.arena), total);
+        if (e == cudaErrorMemoryAllocation && !last) {
+            cudaGetLastError();  // (not an error of this call)
+            sc.arena = nullptr;
+            continue;
+        }
+        if (e == cudaSuccess) e = cudaMemset(sc.arena, 0, total);
+        if (e != cudaSuccess) rc = cuda_fail(e, "vbd_solver_create: self-contact scratch");
+    }
     if (!rc)
         for (const auto& p : placed) *p.first = sc.arena + p.second;
     if (!rc && V > 0) {
