@@ -27,6 +27,13 @@ def _folded(n=24, side=0.5, gap=0.003):
     return model, q.astype(np.float32)
 
 
+def _around(x, n=24, rings=2):
+    """The largest value within two rows and columns of each vertex of the n x n cloth."""
+    padded = np.pad(x.reshape(n, n), rings)
+    shifts = [padded[r:r + n, c:c + n] for r in range(2 * rings + 1) for c in range(2 * rings + 1)]
+    return np.max(shifts, axis=0).reshape(-1)
+
+
 def test_rows_beyond_the_rank_sort_are_ordered():
     model, q = _folded()
     solver = SolverVBD(model, iterations=1, particle_enable_self_contact=True, particle_self_contact_radius=RADIUS,
@@ -74,11 +81,12 @@ def test_tables_within_and_beyond_their_capacity(margin, beyond):
         solver.step(a, b, None, None, DT)
         _, q_ref, _ = orc.step(q_in, qd_in, None, DT, 5)
         _, q_64, _ = exact.step(q_in, qd_in, None, DT, 5)
-        # the parity tolerance of a step, and where pushing out of the 3 mm overlap is ill-conditioned
-        # (a wider margin lets vertices move farther in one step), what FP32 itself is off by: four
-        # times the FP32 oracle's distance from the FP64 one
-        bound = 1e-5 + 4.0 * np.abs(q_ref - q_64).max()
-        assert np.abs(b.particle_q.cpu().numpy() - q_ref).max() <= bound
+        # the parity tolerance of a step, and at vertices where pushing out of the 3 mm overlap is
+        # ill-conditioned (a wider margin lets them move farther in one step), what FP32 itself is off by:
+        # four times the FP32 oracle's distance from the FP64 one at the vertex or two rings around it,
+        # but never more than 1% of the radius (a missing contact moves a vertex by 1 mm and more)
+        bound = np.minimum(1e-5 + 4.0 * _around(np.abs(q_ref - q_64).max(axis=1)), 0.01 * RADIUS)
+        assert (np.abs(b.particle_q.cpu().numpy() - q_ref).max(axis=1) <= bound).all()
         a, b = b, a
     st = solver.status()
     assert st["self_contact_overflow"] == 0 and st["nonfinite_updates"] == 0
