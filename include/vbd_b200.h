@@ -126,8 +126,8 @@ typedef struct VbdSolverOptions {
     int32_t iterations;           /* default VBD iterations per step (reference default 10) */
     float friction_epsilon;       /* reference default 1e-2 */
     int32_t lanes_per_vertex;     /* 1,2,4,8,16 = that many lanes cooperate on one vertex; 0 = default: 16
-                                     or 8 for models without worlds whose largest color has at most 4,096 or
-                                     10,240 vertices, else 4 (vbd_solver_info reports it);
+                                     or 8 for models without worlds whose largest color has at most 4,144 or
+                                     8,288 vertices, else 4 (vbd_solver_info reports it);
                                      -1 = record-parallel sweep (one thread per element record) */
     int32_t block_size;           /* threads per block of the sweep, 0 = default 128 (64/128/256 when
                                      lanes_per_vertex is 0) */

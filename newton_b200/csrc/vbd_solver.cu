@@ -1031,7 +1031,8 @@ __global__ void __launch_bounds__(256, kCap ? 4 : 1) sweep_kernel(SweepArgs a) {
 // plain sweep: at 74 (what the compiler picks for the extra reduction) the allocation rounds up
 // to 80 registers per thread, two color grids no longer fit on an SM together, and each launch
 // loses its overlap with the previous one.
-// (16 lanes: small grids, and the pair walk needs more.)
+// (16 lanes: not held to 72.  The pair walk takes 77 to 80 registers in the gate's and the damped staged
+// sweep, so a color's grid overlaps the one before it up to 3,552 vertices instead of 4,144.)
 constexpr int sweep_registers(int L) { return L == 16 ? 112 : 72; }
 
 template <int L, int kDamp, bool kStaged = false>
@@ -2044,17 +2045,23 @@ static const char* launch_shape_error(int lanes, int block) {
 }
 
 // Lanes per vertex when the caller leaves the choice to the library.  A small color is a latency chain
-// over a vertex's records, and more lanes shorten it while the GPU has room: 10 iterations take, in
-// us with 4 / 8 / 16 lanes, 208 / 172 / 150 at 1,024 vertices, 240 / 193 / 178 at 9,216, 237 / 203 / 196
-// at 16,384 (4,096 per color), 232 / 197 / 207 at 22,500, 269 / 256 / 240 at 32,761 and, where 4
-// lanes fill it, 304 / 301 / 402 at 65,536, 465 / 597 / 824 at 129,600.
+// over a vertex's records, and more lanes shorten it while a launch's blocks still find room beside those
+// of the launch before it: two color grids on the GPU together, at seven blocks of 128 threads per SM.
+// 10 iterations on the draped cloth, in us with 4 / 8 / 16 lanes (the line 16 | 8 lies at 4,144 vertices of a
+// color, 8 | 4 at 8,288):
+//   largest color   3,364           4,096           4,225           7,396           8,281           8,464
+//   plain           205/184/158     203/190/173     209/201/215     218/210/230     224/222/227     225/256/238
+//   gated           289/268/240     286/273/277     289/271/284     304/291/332     306/302/338     305/316/340
+// (the gate's 16-lane sweep takes more registers, 6 blocks per SM, and loses its lead at 3,552; it keeps
+// the plain step's lane count, so that a gate changes no bits).  Damped curtains: the same lines.
 // A model made of worlds keeps 4: the lane count decides the summation order, and a world's result
 // must not depend on how many others share its model (shards reproduce the whole bit for bit).
 static int default_lanes(const VbdModelImpl& m) {
     if (m.n_worlds > 0) return 4;
     int largest = 0;
     for (int c = 0; c < m.C; ++c) largest = std::max(largest, m.color_start[c + 1] - m.color_start[c]);
-    return largest <= 4096 ? 16 : (largest <= 10240 ? 8 : 4);
+    auto overlaps = [largest](int lanes) { return 2 * ((static_cast<long long>(largest) * lanes + 127) / 128) <= 7 * 148; };
+    return overlaps(16) ? 16 : (overlaps(8) ? 8 : 4);
 }
 
 static bool same_contacts(const VbdContacts& a, const VbdContacts& b) { return std::memcmp(&a, &b, sizeof(a)) == 0; }

@@ -39,3 +39,11 @@ def test_staged_gated_and_plain_sweeps_give_the_same_bits(n, lanes, block, kd):
         results.append(a.particle_q.clone())
     for other in results[1:]:
         assert torch.equal(results[0], other)
+
+
+@pytest.mark.parametrize("n, lanes", [(128, 16), (130, 8), (182, 8), (184, 4)])  # colors of 4,096 / 4,225 / 8,281 / 8,464
+def test_default_lanes_at_the_lines(n, lanes):
+    model, _ = scenes.draped_cloth(n=n, seed=0)
+    largest = max(len(g) for g in model.particle_color_groups)
+    assert (largest <= 4144) == (lanes == 16) and (largest <= 8288) == (lanes >= 8)
+    assert SolverVBD(model).launch_info()["lanes_per_vertex"] == lanes
