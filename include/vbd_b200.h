@@ -236,10 +236,15 @@ int vbd_step(VbdSolver* solver, float* q_in, const float* qd_in, const float* f_
              float* qd_out, const VbdContacts* contacts, float dt, int32_t iterations, void* stream);
 
 /* Batched step of `count` independent solvers (each with its own model and state) in one call:
- * element b of every array is solver b's argument to vbd_step, and the steps are enqueued in
- * order on `stream`, so the results are those of `count` vbd_step calls.  f_ext and contacts may
- * be NULL as a whole (no external force / no contacts for every solver) or hold NULL entries;
- * iterations may be NULL (every solver's default) or hold one count per solver (< 0: default).
+ * element b of every array is solver b's argument to vbd_step, and the results are those of `count`
+ * vbd_step calls in order on `stream`.  Distinct solvers of at most 65,536 particles without a
+ * resident plan, none writing what another one reads or writes, run beside one another on streams
+ * of their own, after everything enqueued on `stream` and before what follows on it; else, and
+ * inside the caller's stream capture, the steps are enqueued in order.  (The first call with new
+ * arrays captures each solver's step graph on the host, one after the other, which hides that.)
+ * f_ext and contacts may be NULL as a whole (no external force / no contacts for every solver) or
+ * hold NULL entries; iterations may be NULL (every solver's default) or hold one count per solver
+ * (< 0: default).
  * The reference batches by putting several worlds in one Model (ModelBuilder.add_world), which
  * vbd_model_create supports directly and which is the faster layout for many small cloths (one
  * launch per color for all worlds); this entry point is for models that cannot be merged.

@@ -12,7 +12,11 @@
 //   that the next epilogue waits for)
 // Rounding is that of a layer-by-layer BF16 pass: weights, inputs, activations, pre-activations (for
 // silu') and gradients are rounded to BF16 as operands, every product accumulates in FP32, and
-// biases, SiLU and its derivative are FP32.
+// biases, SiLU and its derivative are FP32 -- with the approximate FP32 division (__fdividef, 2 ulp) in the
+// sigmoid, and the bias gradients summed by the tensor cores.  Against 64 bits over 1,000 to 131,072
+// samples (42 passes) the gradients are off by 2.5599e-3 on average, at most 3.7793e-3; with the IEEE
+// division 2.5599e-3 and 3.7810e-3 (and 64 us instead of 45), and the mma.sync passes 2.5599e-3 and
+// 3.7807e-3.
 //
 // Operand views.  A tile operand of 128 rows by K columns is stored K-major without swizzle (as in
 // vbd_mlp_tc.cuh): core matrices of 8 rows x 16 bytes, 8-row groups 128 bytes apart, groups of 8

@@ -29,11 +29,12 @@
 //   * forces are gathered per vertex of the current color, one warp per vertex taking its entries
 //     round-robin in a fixed order (own vertex-triangle pairs, then the pairs of each incident
 //     triangle, then the edge-edge pairs of each incident edge) and reduced with xor shuffles, so
-//     results are deterministic;
+//     results are deterministic (while no buffer overflows: below);
 //   * truncation ratios are reduced with an integer atomicMin on the (non-negative) float bits,
 //     which is exact and order-independent.
 // Buffers are fixed-size (reference defaults: 32 triangles per vertex, 64 edges per edge; plus
-// 32 vertices per triangle for the gather); candidates beyond a buffer are dropped and counted.
+// 32 vertices per triangle for the gather); candidates beyond a buffer are dropped and counted.  Which
+// ones a full row keeps depends on scheduling, so runs repeat bit for bit only while the count is zero.
 #include "vbd_self_contact.h"
 
 #include <cub/device/device_scan.cuh>
@@ -261,7 +262,7 @@ constexpr int kVtLanes = 4;  // lanes per vertex-triangle query (one lane: 1.49 
 // distance comes before the filters: most queued pairs are neighbours in the same layer, farther
 // apart than the margin, and the ring filter walks a list.  Accepted partners are appended to their
 // rows through atomic slots; sort_rows_kernel then orders every row, so the lists do not depend on
-// scheduling.  On the folded 1.05 M vertex cloth: edge query 4.59 -> 2.59 ms, vertex query 2.31 -> 1.21 ms.
+// scheduling, but for a row that met more partners than it holds (counted).  On the folded 1.05 M vertex cloth: edge query 4.59 -> 2.59 ms, vertex query 2.31 -> 1.21 ms.
 struct PairQueue {
     int2* slots;  // this warp's 64 entries in shared memory
     int n;        // (warp-uniform)

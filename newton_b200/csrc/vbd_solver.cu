@@ -2320,7 +2320,8 @@ struct Ends {
 
 // Models of at most this many particles leave most of the GPU idle in every sweep, so the steps of
 // different solvers run beside one another: 16 steps of 1,024 vertices 2,050 -> 194 us, 4 of 16,384
-// 655 -> 330, 4 of 65,536 1,064 -> 613.
+// 655 -> 330, 4 of 65,536 1,064 -> 613 (replayed; the first call with new arrays captures each solver's
+// graph on the host, one after the other: 8 steps of 400 to 2,304 vertices 2,297 -> 2,049).
 constexpr int kConcurrentParticles = 65536;
 
 // Whether the entries of a batch may run beside one another: distinct solvers on one device, small
